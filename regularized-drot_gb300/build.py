@@ -1,7 +1,8 @@
 """Build recipe of the solver library (libdrot_gb300.so) for sm_103a.
 
 nvcc compiles the translation units csrc/drot_api.cu (single-instance
-solver and C ABI), csrc/drot_batch.cu (batched solver) and
+solver and C ABI), csrc/drot_resident.cu (the single-instance solve of a
+problem that fits the chip), csrc/drot_batch.cu (batched solver),
 csrc/drot_adjoint.cu (implicit QR adjoint), csrc/drot_gl_adjoint.cu
 (unrolled GL adjoint) and csrc/drot_cost.cu (tensor-core cost matrices) in
 parallel and links them into
@@ -23,7 +24,7 @@ CSRC = os.path.join(PKG, "csrc")
 INCLUDE = os.path.join(REPO, "include")
 OUT = os.path.join(PKG, "reg_drot", "libdrot_gb300.so")
 SOURCES = [os.path.join(CSRC, f)
-           for f in ("drot_api.cu", "drot_batch.cu", "drot_adjoint.cu",
+           for f in ("drot_api.cu", "drot_resident.cu", "drot_batch.cu", "drot_adjoint.cu",
                      "drot_gl_adjoint.cu", "drot_cost.cu")]
 DEPS = SOURCES + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))] + \
     [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE)]

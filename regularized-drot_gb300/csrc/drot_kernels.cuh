@@ -467,6 +467,12 @@ __device__ __forceinline__ f32x2 x2_div_rn_by_fma(f32x2 a, f32x2 nb, f32x2 y) {
   return x2_fma(r1, y, q1);
 }
 
+// div_rn_two on both lanes.
+__device__ __forceinline__ f32x2 x2_div_rn_two(f32x2 a, f32x2 nb, f32x2 y) {
+  const f32x2 q0 = x2_mul(a, y);
+  return x2_fma(x2_fma(nb, q0, a), y, q0);
+}
+
 template <int VEC>
 __device__ __forceinline__ void load_vec(const float* ptr, float (&v)[VEC]) {
   if constexpr (VEC == 4) {

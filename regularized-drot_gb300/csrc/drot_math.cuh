@@ -49,6 +49,22 @@ DROT_HD float div_rn_by_fma(float a, float b, float y) {
   return fmaf(r1, y, q1);
 }
 
+// Whether q0 = RN(a*y) lies within one ulp of a / b for every a, so that the
+// theorem applies to it and the first correction already gives RN(a/b):
+// |q0 - a/b| <= 1/2 ulp + (a/b) |b*y - 1| < 1/2 ulp + 2^24 |b*y - 1| ulp.
+// True for all but about one divisor in 300 close to 1 (|b*y - 1| is at most
+// b 2^-25).
+inline bool div_two_step_exact(float b, float y) {
+  return fabs((double)b * (double)y - 1.0) <= 0.49 * 5.9604644775390625e-8;  // 0.49 * 2^-24
+}
+
+// The short sequence, for divisors that pass div_two_step_exact and the
+// dividends of div_rn_by_fma.
+DROT_HD float div_rn_two(float a, float b, float y) {
+  const float q0 = a * y;
+  return fmaf(fmaf(-b, q0, a), y, q0);
+}
+
 // a / b correctly rounded, for b > 0 finite and y == RN(1/b).  Zero takes
 // the FMA path too (every step is exact); only nonzero dividends below 2^-90
 // use the plain division.
