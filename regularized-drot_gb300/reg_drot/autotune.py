@@ -53,8 +53,11 @@ def clear():
 
 def _candidates(kind, aligned, fp32):
     kvs = (1, 2, 4) if kind == "qr" else (1, 2, 4, 8)
-    out = [dict(vectors_per_lane=kv, warps_per_cta=w, data_path=0, ctas_per_sm=0)
-           for kv in kvs for w in (4, 8, 16)]
+    # the planner's own choice (for problems that fit the chip the resident
+    # kernel, which no other candidate selects), then the streaming shapes
+    out = [dict(vectors_per_lane=0, warps_per_cta=0, data_path=0, ctas_per_sm=0)]
+    out += [dict(vectors_per_lane=kv, warps_per_cta=w, data_path=0, ctas_per_sm=0)
+            for kv in kvs for w in (4, 8, 16)]
     if aligned and fp32:
         out += [dict(vectors_per_lane=kv, warps_per_cta=w, data_path=1, ctas_per_sm=ct)
                 for kv in kvs for w in (8, 16) for ct in (1, 2)]
