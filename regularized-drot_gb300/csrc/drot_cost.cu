@@ -251,23 +251,32 @@ static size_t cost_smem_bytes(int dim) {
 // For G = dL/dC of one instance (column-major m x n, the layout of C),
 //     dL/dx_i = 2 scale (x_i sum_j G_ij - sum_j G_ij y_j)
 //     dL/dy_j = 2 scale (y_j sum_i G_ij - sum_i G_ij x_i)
-// (G zeroed where C = 0 when the cost was clamped).  CTA (band b, instance
-// k) owns rows [256 b, 256 b + 256) and walks the columns in tiles of 64:
-// the G tile goes to shared memory (row pitch 65: conflict-free both ways),
-// thread t accumulates row t's sums over the columns (its dL/dx, written at
-// the end), and thread (column c, k-group) the column sums of the tile over
-// the band's rows, written as the band's partial of dL/dy; a second kernel
-// adds the bands' partials in band order.  No atomics: deterministic.
+// (G zeroed where C = 0 when the cost was clamped).  A CTA takes a block of
+// 256 rows (band) by a few 32-column tiles (chunk) of one instance; thread t loads 4 rows (t % 64) of the 8 columns t / 64 + 4 p of a
+// tile into registers (128-bit loads, 8 of G and 8 of C in flight).
+//   rows: from the registers, 4 rows x (d + 1) sums per thread with y of the
+//     column broadcast from shared memory (d / 4 loads for 4 (d + 1) FMAs);
+//     the four column groups' sums are added at the end -> the chunk's partial
+//     of dL/dx.
+//   columns: the tile goes to shared memory column by column (pitch 260
+//     floats: conflict-free 128-bit accesses both ways); a thread sums 8 of
+//     the d components of two columns over its share of the band's rows (x
+//     broadcast), the shares are added -> the band's partial of dL/dy.
+// A second kernel adds the partials in order.  No atomics: deterministic.
+// Bound by the FP32 pipe (2 (d + 1) FMAs per element) and the 8 B per element
+// of G and C about alike at d = 16.  One CTA per band walking all columns,
+// which this replaces, kept 16 CTAs busy on a 4000 x 3000 matrix: 900 us
+// against 47 us here.
 
-constexpr int kGradRows = 256;  // rows per CTA (= threads)
-constexpr int kGradCols = 64;   // columns per tile
-constexpr int kGradPitch = kGradCols + 1;
+constexpr int kGradRows = 256;   // rows per band (= threads)
+constexpr int kGradCols = 32;    // columns per tile
+constexpr int kGradPitch = kGradRows + 4;
 
 struct GradInst {
   long long x_off, y_off, c_off;  // element offsets: x (m x d), y (n x d), G / C (ld x n)
-  long long part_off;             // float offset of its partials [bands][n][d + 1]
-  int m, n, ld, bands, aligned;
-  int pad;
+  long long py_off, px_off;       // float offsets of its partials: [bands][n][d + 1] of dL/dy,
+                                  // [chunks][m][d + 1] of dL/dx
+  int m, n, ld, bands, chunks, aligned;
 };
 
 struct GradParams {
@@ -279,131 +288,259 @@ struct GradParams {
   float* gy;
   float* part;
   int n_inst;
+  int chunk_cols;  // columns of a chunk (whole tiles)
   float scale2;  // 2 * scale
   GradInst inst[kCostMaxInst];
 };
 
+// Shared memory of the kernel (floats): the tile, x of the band, y of the
+// tile, the column shares; the row groups' sums reuse the tile.
 template <int DIM>
-__global__ void __launch_bounds__(kGradRows, 2) cost_grad_kernel(const GradParams P) {
+struct GradShape {
+  static constexpr int KS = DIM / 8;          // component slices of a column pair
+  static constexpr int RG = KS == 3 ? 4 : 16 / KS;  // row shares of 16 column pairs x KS
+  static constexpr int TILE = kGradCols * kGradPitch;
+  static constexpr int XS = kGradRows * DIM, YS = kGradCols * DIM;
+  static constexpr int SHARE = RG * kGradCols * (DIM + 1);
+  static constexpr int GROUP = kGradRows * (DIM + 1);  // one column group's row sums
+  static constexpr int FLOATS = (TILE > GROUP ? TILE : GROUP) + XS + YS + SHARE;
+};
+
+template <int DIM>
+__global__ void __launch_bounds__(kGradRows, DIM <= 16 ? 2 : 1)
+cost_grad_kernel(const __grid_constant__ GradParams P) {
+  using S = GradShape<DIM>;
   extern __shared__ __align__(16) float gsm[];
-  float* gt = gsm;                               // [kGradRows][kGradPitch]
-  float* xs = gt + kGradRows * kGradPitch;       // [kGradRows][DIM]
-  float* ys = xs + kGradRows * DIM;              // [kGradCols][DIM]
-  const GradInst I = P.inst[blockIdx.y];
-  const int b = blockIdx.x;
-  if (b >= I.bands) return;
+  float* const gt = gsm;  // [kGradCols][kGradPitch]
+  float* const xs = gsm + (S::TILE > S::GROUP ? S::TILE : S::GROUP);  // [kGradRows][DIM]
+  float* const ys = xs + S::XS;                                       // [kGradCols][DIM]
+  float* const sh = ys + S::YS;                                       // [RG][kGradCols][DIM + 1]
+  const GradInst& I = P.inst[blockIdx.z];
+  const int band = blockIdx.x;
+  if (band >= I.bands || (int)blockIdx.y >= I.chunks) return;
   const int t = threadIdx.x;
-  const int r0 = b * kGradRows;
-  constexpr int KG = DIM / 4;  // k values per column thread
-  for (int e = t; e < kGradRows * DIM; e += kGradRows) {
-    const int r = e / DIM, k = e - r * DIM;
-    xs[e] = r0 + r < I.m ? __ldg(P.x + I.x_off + (long long)(r0 + r) * DIM + k) : 0.0f;
-  }
-  float ax[DIM], rs = 0.0f;
+  const int m = I.m, n = I.n;
+  const long long ld = I.ld;
+  const int r0 = band * kGradRows;
+  for (int e = t; e < kGradRows * DIM; e += kGradRows)
+    xs[e] = r0 + e / DIM < m ? __ldg(P.x + I.x_off + (long long)r0 * DIM + e) : 0.0f;
+  const int rr = 4 * (t % 64), cg = t / 64, i = r0 + rr;
+  const float* const gcol = P.g + I.c_off + i;
+  const float* const ccol = P.c ? P.c + I.c_off + i : nullptr;
+  const bool vec = I.aligned && i + 4 <= m;
+  // column phase: pair cp, slice ks, row share rg
+  const int cp = t % 16, ks = (t / 16) % S::KS, rg = t / (16 * S::KS);
+  for (int chunk = blockIdx.y; chunk < I.chunks; chunk += gridDim.y) {
+    const int cb = chunk * P.chunk_cols, ce = min(cb + P.chunk_cols, n);
+    float ax[4][DIM], rs[4];
 #pragma unroll
-  for (int k = 0; k < DIM; ++k) ax[k] = 0.0f;
-  const int cc = t % kGradCols, kg = t / kGradCols;
-  const float* gbase = P.g + I.c_off;
-  const float* cbase = P.c ? P.c + I.c_off : nullptr;
-  for (int c0 = 0; c0 < I.n; c0 += kGradCols) {
-    __syncthreads();  // the previous tile's readers are done
-    for (int e = t; e < kGradCols * DIM; e += kGradRows) {
-      const int c = e / DIM, k = e - c * DIM;
-      ys[e] = c0 + c < I.n ? __ldg(P.y + I.y_off + (long long)(c0 + c) * DIM + k) : 0.0f;
+    for (int e = 0; e < 4; ++e) {
+      rs[e] = 0.0f;
+#pragma unroll
+      for (int k = 0; k < DIM; ++k) ax[e][k] = 0.0f;
     }
-    // G tile: a column is 256 contiguous rows; 64 threads per column, 4 rows each.
-    for (int pass = 0; pass < kGradCols / 4; ++pass) {
-      const int c = pass * 4 + t / 64, rr = 4 * (t % 64);
-      const int j = c0 + c, i = r0 + rr;
-      float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      if (j < I.n && i < I.m) {
-        const long long off = (long long)j * I.ld + i;
-        if (I.aligned && i + 4 <= I.m) {
-          const float4 q = __ldg(reinterpret_cast<const float4*>(gbase + off));
-          v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-          if (cbase) {
-            const float4 cq = __ldg(reinterpret_cast<const float4*>(cbase + off));
-            v[0] = cq.x > 0.0f ? v[0] : 0.0f;
-            v[1] = cq.y > 0.0f ? v[1] : 0.0f;
-            v[2] = cq.z > 0.0f ? v[2] : 0.0f;
-            v[3] = cq.w > 0.0f ? v[3] : 0.0f;
-          }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            if (i + e < I.m) {
-              const float gv = __ldg(gbase + off + e);
-              v[e] = (!cbase || __ldg(cbase + off + e) > 0.0f) ? gv : 0.0f;
-            }
+    for (int c0 = cb; c0 < ce; c0 += kGradCols) {
+      float v[8][4];
+      {
+        // the next tile's lines into L2: this tile's loads then wait for L2,
+        // not for DRAM (32 columns of 8 lines each, of G and of C)
+        const int jn = c0 + kGradCols + t / 8, ln = r0 + 32 * (t % 8);
+        if (jn < n && ln < m) {
+          prefetch_l2(P.g + I.c_off + (long long)jn * ld + ln);
+          if (P.c) prefetch_l2(P.c + I.c_off + (long long)jn * ld + ln);
         }
       }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) gt[(rr + e) * kGradPitch + c] = v[e];
+      for (int hb = 0; hb < 8; hb += 4) {
+        float cv[4][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            v[hb + q][e] = 0.0f;
+            cv[q][e] = 1.0f;
+          }
+        }
+        if (vec) {
+          // all loads of the half tile before the first use
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int j = c0 + cg + 4 * (hb + q);
+            if (j < ce) load_vec_nc<4>(gcol + (long long)j * ld, v[hb + q]);
+          }
+          if (ccol) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int j = c0 + cg + 4 * (hb + q);
+              if (j < ce) load_vec_nc<4>(ccol + (long long)j * ld, cv[q]);
+            }
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int j = c0 + cg + 4 * (hb + q);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (j < ce && i + e < m) {
+                v[hb + q][e] = __ldg(gcol + (long long)j * ld + e);
+                if (ccol) cv[q][e] = __ldg(ccol + (long long)j * ld + e);
+              }
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[hb + q][e] = cv[q][e] > 0.0f ? v[hb + q][e] : 0.0f;
+      }
+      __syncthreads();  // the previous tile's readers are done
+#pragma unroll
+      for (int p = 0; p < 8; ++p)
+        store_vec<4>(gt + (cg + 4 * p) * kGradPitch + rr, v[p]);
+      for (int e = t; e < kGradCols * DIM; e += kGradRows)
+        ys[e] = c0 + e / DIM < ce ? __ldg(P.y + I.y_off + (long long)c0 * DIM + e) : 0.0f;
+      __syncthreads();
+#pragma unroll
+      for (int p = 0; p < 8; ++p) {
+        const float* const yp = ys + (cg + 4 * p) * DIM;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) rs[e] += v[p][e];
+#pragma unroll
+        for (int k = 0; k < DIM; k += 4) {
+          const float4 y4 = *reinterpret_cast<const float4*>(yp + k);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            ax[e][k] = fmaf(v[p][e], y4.x, ax[e][k]);
+            ax[e][k + 1] = fmaf(v[p][e], y4.y, ax[e][k + 1]);
+            ax[e][k + 2] = fmaf(v[p][e], y4.z, ax[e][k + 2]);
+            ax[e][k + 3] = fmaf(v[p][e], y4.w, ax[e][k + 3]);
+          }
+        }
+      }
+      if (rg < S::RG) {
+        float ay[2][8], cs[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int k = 0; k < 8; ++k) ay[0][k] = ay[1][k] = 0.0f;
+        constexpr int SPAN = kGradRows / S::RG;
+#pragma unroll 2
+        for (int r = rg * SPAN; r < (rg + 1) * SPAN; r += 4) {
+          const float4 ga = *reinterpret_cast<const float4*>(gt + cp * kGradPitch + r);
+          const float4 gb = *reinterpret_cast<const float4*>(gt + (cp + 16) * kGradPitch + r);
+          const float a4[4] = {ga.x, ga.y, ga.z, ga.w}, b4[4] = {gb.x, gb.y, gb.z, gb.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float* const xp = xs + (r + e) * DIM + ks * 8;
+            const float4 u = *reinterpret_cast<const float4*>(xp);
+            const float4 w = *reinterpret_cast<const float4*>(xp + 4);
+            const float x8[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
+            cs[0] += a4[e];
+            cs[1] += b4[e];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              ay[0][k] = fmaf(a4[e], x8[k], ay[0][k]);
+              ay[1][k] = fmaf(b4[e], x8[k], ay[1][k]);
+            }
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          float* const s = sh + (rg * kGradCols + cp + 16 * q) * (DIM + 1);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) s[ks * 8 + k] = ay[q][k];
+          if (ks == 0) s[DIM] = cs[q];
+        }
+      }
+      __syncthreads();
+      {
+        // the band's partials of the tile's columns (contiguous in memory)
+        const int live = min(kGradCols, ce - c0) * (DIM + 1);
+        float* const pp = P.part + I.py_off + ((long long)band * n + c0) * (DIM + 1);
+        for (int e = t; e < live; e += kGradRows) {
+          float s = sh[e];
+#pragma unroll
+          for (int q = 1; q < S::RG; ++q) s += sh[q * kGradCols * (DIM + 1) + e];
+          pp[e] = s;
+        }
+      }
+    }
+    // the column groups' row sums, one group after the other
+    float* const acc = gsm;  // [kGradRows][DIM + 1]
+    for (int q = 0; q < 4; ++q) {
+      __syncthreads();
+      if (cg == q) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float* const a = acc + (rr + e) * (DIM + 1);
+#pragma unroll
+          for (int k = 0; k < DIM; ++k) a[k] = q ? a[k] + ax[e][k] : ax[e][k];
+          a[DIM] = q ? a[DIM] + rs[e] : rs[e];
+        }
+      }
     }
     __syncthreads();
-    // row t: sums over the tile's columns
-    {
-      const float* grow = gt + t * kGradPitch;
-#pragma unroll 4
-      for (int c = 0; c < kGradCols; ++c) {
-        const float gv = grow[c];
-        rs += gv;
-#pragma unroll
-        for (int k = 0; k < DIM; ++k) ax[k] = fmaf(gv, ys[c * DIM + k], ax[k]);
-      }
-    }
-    // column cc, k-group kg: sums over the band's rows -> the band's partial
-    {
-      float ay[KG], cs = 0.0f;
-#pragma unroll
-      for (int k = 0; k < KG; ++k) ay[k] = 0.0f;
-#pragma unroll 4
-      for (int r = 0; r < kGradRows; ++r) {
-        const float gv = gt[r * kGradPitch + cc];
-        cs += gv;
-#pragma unroll
-        for (int k = 0; k < KG; ++k) ay[k] = fmaf(gv, xs[r * DIM + kg * KG + k], ay[k]);
-      }
-      const int j = c0 + cc;
-      if (j < I.n) {
-        float* pp = P.part + I.part_off + ((long long)b * I.n + j) * (DIM + 1);
-#pragma unroll
-        for (int k = 0; k < KG; ++k) pp[kg * KG + k] = ay[k];
-        if (kg == 0) pp[DIM] = cs;
-      }
-    }
-  }
-  const int i = r0 + t;
-  if (i < I.m) {
-    float* o = P.gx + I.x_off + (long long)i * DIM;
-#pragma unroll
-    for (int k = 0; k < DIM; ++k) o[k] = P.scale2 * fmaf(xs[t * DIM + k], rs, -ax[k]);
+    const int live = min(kGradRows, m - r0) * (DIM + 1);
+    float* const pp = P.part + I.px_off + ((long long)chunk * m + r0) * (DIM + 1);
+    for (int e = t; e < live; e += kGradRows) pp[e] = acc[e];
+    __syncthreads();  // before the next chunk's tiles
   }
 }
 
-// dL/dy_j from the bands' partials, added in band order.
+// dL/dx_i from the chunks' partials and dL/dy_j from the bands', added in
+// order; a thread per component.
 template <int DIM>
-__global__ void cost_grad_reduce_kernel(const GradParams P) {
-  const GradInst I = P.inst[blockIdx.y];
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < I.n; j += gridDim.x * blockDim.x) {
-    float a[DIM + 1];
-#pragma unroll
-    for (int k = 0; k <= DIM; ++k) a[k] = 0.0f;
-    for (int b = 0; b < I.bands; ++b) {
-      const float* pp = P.part + I.part_off + ((long long)b * I.n + j) * (DIM + 1);
-#pragma unroll
-      for (int k = 0; k <= DIM; ++k) a[k] += __ldcg(pp + k);
+__global__ void cost_grad_reduce_kernel(const __grid_constant__ GradParams P) {
+  const GradInst& I = P.inst[blockIdx.y];
+  const long long step = (long long)gridDim.x * blockDim.x;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+       e < (long long)(I.m + I.n) * DIM; e += step) {
+    const bool is_x = e < (long long)I.m * DIM;
+    const long long o = is_x ? e : e - (long long)I.m * DIM;
+    const long long pt = o / DIM;
+    const int k = (int)(o - pt * DIM);
+    const int parts = is_x ? I.chunks : I.bands, count = is_x ? I.m : I.n;
+    const float* pp = P.part + (is_x ? I.px_off : I.py_off) + pt * (DIM + 1);
+    float a = 0.0f, s = 0.0f;
+#pragma unroll 4
+    for (int b = 0; b < parts; ++b, pp += (long long)count * (DIM + 1)) {
+      a += __ldcg(pp + k);
+      s += __ldcg(pp + DIM);
     }
-    const float* yj = P.y + I.y_off + (long long)j * DIM;
-    float* o = P.gy + I.y_off + (long long)j * DIM;
-#pragma unroll
-    for (int k = 0; k < DIM; ++k) o[k] = P.scale2 * fmaf(__ldg(yj + k), a[DIM], -a[k]);
+    const float v = __ldg((is_x ? P.x + I.x_off : P.y + I.y_off) + o);
+    (is_x ? P.gx + I.x_off : P.gy + I.y_off)[o] = P.scale2 * fmaf(v, s, -a);
   }
 }
 
 static size_t grad_smem_bytes(int dim) {
-  return sizeof(float) * ((size_t)kGradRows * kGradPitch + (size_t)kGradRows * dim +
-                          (size_t)kGradCols * dim);
+  return sizeof(float) * (size_t)(dim == 8 ? GradShape<8>::FLOATS
+                                  : dim == 16 ? GradShape<16>::FLOATS
+                                  : dim == 24 ? GradShape<24>::FLOATS : GradShape<32>::FLOATS);
+}
+
+// Tiles per chunk: the CTAs fill whole waves as nearly as they can (every tile
+// costs about the same; a chunk's start about 0.7 of one).  4000 x 3000, d =
+// 16: 5 tiles, 304 CTAs in one wave.
+static int grad_chunk_tiles(int n_inst, const drot_cost_instance* inst, int dim) {
+  int dev = 0, sms = 152;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    sms = 152;
+  }
+  const long long slots = (dim <= 16 ? 2LL : 1LL) * sms;
+  int best = 1;
+  double best_cost = 0.0;
+  for (int k = 1; k <= 64; ++k) {
+    long long ctas = 0;
+    for (int q = 0; q < n_inst; ++q) {
+      const long long tiles = ((long long)inst[q].n + kGradCols - 1) / kGradCols;
+      ctas += ((long long)inst[q].m + kGradRows - 1) / kGradRows * ((tiles + k - 1) / k);
+    }
+    const double cost = (double)((ctas + slots - 1) / slots) * (k + 0.7);
+    if (k == 1 || cost < best_cost) {
+      best = k;
+      best_cost = cost;
+    }
+  }
+  return best;
 }
 
 // Partials layout; returns the floats they need (0: invalid descriptors).
@@ -413,20 +550,28 @@ static long long grad_layout(int n_inst, const drot_cost_instance* inst, int dim
     const drot_cost_instance& a = inst[k];
     if (a.m <= 0 || a.n <= 0 || a.ld < a.m || a.x_offset < 0 || a.y_offset < 0 || a.c_offset < 0)
       return 0;
+  }
+  const int chunk_cols = kGradCols * grad_chunk_tiles(n_inst, inst, dim);
+  if (P) P->chunk_cols = chunk_cols;
+  for (int k = 0; k < n_inst; ++k) {
+    const drot_cost_instance& a = inst[k];
     const int bands = (a.m + kGradRows - 1) / kGradRows;
+    const int chunks = (a.n + chunk_cols - 1) / chunk_cols;
     if (P) {
       GradInst& I = P->inst[k];
       I.x_off = a.x_offset * dim;
       I.y_off = a.y_offset * dim;
       I.c_off = a.c_offset;
-      I.part_off = part;
+      I.py_off = part;
+      I.px_off = part + (long long)bands * a.n * (dim + 1);
       I.m = a.m;
       I.n = a.n;
       I.ld = a.ld;
       I.bands = bands;
+      I.chunks = chunks;
       I.aligned = (a.ld % 4 == 0) && (a.c_offset % 4 == 0);
     }
-    part += (long long)bands * a.n * (dim + 1);
+    part += ((long long)bands * a.n + (long long)chunks * a.m) * (dim + 1);
   }
   return part;
 }
@@ -461,10 +606,12 @@ int drot_sqeuclidean_cost_grad(int n_inst, const drot_cost_instance* inst, const
   const long long nf = grad_layout(n_inst, inst, dim, &P);
   if (nf <= 0) return DROT_ERR_INVALID_ARG;
   if (workspace_bytes < (size_t)nf * sizeof(float)) return DROT_ERR_WORKSPACE;
-  int max_bands = 0, max_n = 0;
+  int max_bands = 0, max_chunks = 0;
+  long long max_points = 0;
   for (int k = 0; k < n_inst; ++k) {
     max_bands = std::max(max_bands, P.inst[k].bands);
-    max_n = std::max(max_n, P.inst[k].n);
+    max_chunks = std::max(max_chunks, P.inst[k].chunks);
+    max_points = std::max(max_points, (long long)P.inst[k].m + P.inst[k].n);
   }
   P.x = x;
   P.y = y;
@@ -489,10 +636,11 @@ int drot_sqeuclidean_cost_grad(int n_inst, const drot_cost_instance* inst, const
       cudaSuccess)
     return DROT_ERR_CUDA;
   void* args[] = {(void*)&P};
-  if (cudaLaunchKernel(k1, dim3(max_bands, n_inst), dim3(kGradRows), args, smem, st) !=
+  if (cudaLaunchKernel(k1, dim3(max_bands, std::min(max_chunks, 65535), n_inst), dim3(kGradRows), args, smem, st) !=
           cudaSuccess ||
-      cudaLaunchKernel(k2, dim3(std::min((max_n + 255) / 256, 64), n_inst), dim3(256), args, 0,
-                       st) != cudaSuccess) {
+      cudaLaunchKernel(k2, dim3((unsigned)std::min<long long>((max_points * dim + 255) / 256, 608),
+                                n_inst), dim3(256),
+                       args, 0, st) != cudaSuccess) {
     cudaGetLastError();
     return DROT_ERR_CUDA;
   }
