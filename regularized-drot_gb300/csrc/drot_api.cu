@@ -558,6 +558,7 @@ struct SolveArgs {
   cudaStream_t stream;
   const int* bounds = nullptr;  // GL: caller's group boundaries (null: the reference's)
   int stop_every = 0, stop_le = 0;  // numpy-API stop rule (QR)
+  int first = 0;  // iterations before this call, where that is known
 };
 
 static int read_stats(const void* ws, drot_result* r, cudaStream_t stream) {
@@ -665,6 +666,7 @@ static int run_solve(const SolveArgs& A, drot_result* result) {
   prm.nc_rcp = (float)(1.0 / (double)(float)A.nc);
   prm.nr_rcp = (float)(1.0 / (double)(float)A.nr);
   prm.max_iters = A.max_iters;
+  prm.first = A.first;
   prm.stop_every = A.stop_every;
   prm.stop_le = A.stop_le;
   prm.res2_stop = res2_threshold(A.eps, A.mode == MODE_QR && !A.stop_le);
@@ -782,6 +784,19 @@ static StateLayout state_layout(size_t base, int nr, int nc) {
 }
 
 static thread_local int g_last_status = DROT_OK;
+
+// One GL iteration, iteration `index` of a solve's segment (drot_gl_adjoint.cu
+// recomputes a segment one iteration at a time).
+int gl_iteration(const void* c, int c_dtype, const float* p, const float* q, int n_rows,
+                 int n_cols, int n_groups, float step_size, float lambda, int index, float* x,
+                 float* a, float* b, float* phi1, float* phi2, float* alpha, void* workspace,
+                 size_t workspace_bytes, cudaStream_t stream) {
+  if (n_groups <= 0) return DROT_ERR_INVALID_ARG;
+  SolveArgs A = {MODE_GL, c, c_dtype, p, q, n_rows, n_cols, n_groups, step_size, 1.0f, lambda,
+                 1, -1.0f, x, a, b, phi1, phi2, alpha, workspace, workspace_bytes, stream};
+  A.first = index;
+  return run_solve(A, nullptr);
+}
 
 }  // namespace drot
 

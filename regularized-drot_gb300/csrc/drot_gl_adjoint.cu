@@ -45,6 +45,12 @@
 
 namespace drot {
 
+// drot_api.cu: iteration `index` of a segment, the stop test off.
+int gl_iteration(const void* c, int c_dtype, const float* p, const float* q, int n_rows,
+                 int n_cols, int n_groups, float step_size, float lambda, int index, float* x,
+                 float* a, float* b, float* phi1, float* phi2, float* alpha, void* workspace,
+                 size_t workspace_bytes, cudaStream_t stream);
+
 constexpr int kGlaChunk = 16;     // columns per CTA in gl_adj_elems
 constexpr int kGlaRows = 1024;    // rows per CTA in gl_adj_elems
 constexpr int kGlaThreads = 256;
@@ -558,10 +564,9 @@ int drot_gl_adjoint_segment(const void* c, int c_dtype, const float* p, const fl
         cudaMemcpyAsync(s_k + mn + n_rows, phi2, sizeof(float) * n_cols, cudaMemcpyDeviceToDevice,
                         st) != cudaSuccess)
       return DROT_ERR_CUDA;
-    // One GL iteration; eps = -1 never stops it early.
-    const int rc = drot_gl_solve_ex(c, c_dtype, p, q, n_rows, n_cols, n_groups, step_size, lambda,
-                                    1, -1.0f, x, a, b, phi1, phi2, alpha, solve_ws,
-                                    solve_ws_bytes, nullptr, stream);
+    // One GL iteration, the stop test off.
+    const int rc = gl_iteration(c, c_dtype, p, q, n_rows, n_cols, n_groups, step_size, lambda, k,
+                                x, a, b, phi1, phi2, alpha, solve_ws, solve_ws_bytes, st);
     if (rc != DROT_OK) return rc;
   }
   // Reverse steps.

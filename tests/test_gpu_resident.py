@@ -149,3 +149,46 @@ def test_segments_equal_one_launch(cuda, solver_lib):
         out.append(st)
     for k in out[0]:
         assert torch.equal(out[0][k], out[1][k]), k
+
+
+def test_streamed_gl_iterations_recomputed_singly_give_the_same_bits(cuda, solver_lib):
+    """Beyond the chip the streaming kernel alternates the order of its
+    columns; a segment recomputed one iteration at a time
+    (drot_gl_adjoint_segment) ends in the state of one launch over it."""
+    import ctypes
+    from reg_drot._lib import DrotResult
+    nr, nc, G, n = 2600, 2100, 2, 5
+    c, p, q = (t.to(cuda) for t in _problem(nr, nc, 12))
+    s = float(np.float32(2.0) / np.float32(nr + nc))
+    stream = torch.cuda.current_stream().cuda_stream
+    nbytes = solver_lib.drot_gl_workspace_bytes(nr, nc, G)
+    ws = torch.empty(nbytes + 256, dtype=torch.uint8, device=cuda)
+    wptr = ws.data_ptr() + (-ws.data_ptr()) % 256
+    out = []
+    for single in (False, True):
+        st = {"x": torch.empty(nc, nr, device=cuda), "a": torch.empty(nr, device=cuda),
+              "b": torch.empty(nc, device=cuda), "phi1": torch.empty(nr, device=cuda),
+              "phi2": torch.empty(nc, device=cuda), "alpha": torch.empty(1, device=cuda)}
+        ptrs = [t.data_ptr() for t in st.values()]
+        assert solver_lib.drot_init_state(nr, nc, s, 1, p.data_ptr(), q.data_ptr(), *ptrs,
+                                          stream) == 0
+        if single:
+            ab = solver_lib.drot_gl_adjoint_workspace_bytes(nr, nc, G)
+            aws = torch.empty(ab + 256, dtype=torch.uint8, device=cuda)
+            bars = [torch.zeros(k, device=cuda) for k in
+                    (nr * nc, 2 * (nr + nc) + 1, nr * nc, nr, nc)]
+            states = torch.empty(n * (nr * nc + nr + nc), device=cuda)
+            rc = solver_lib.drot_gl_adjoint_segment(
+                c.data_ptr(), 0, p.data_ptr(), q.data_ptr(), nr, nc, G, s, 1e-6, *ptrs, n,
+                states.data_ptr(), wptr, nbytes, *[t.data_ptr() for t in bars],
+                aws.data_ptr() + (-aws.data_ptr()) % 256, ab, stream)
+        else:
+            res = DrotResult()
+            rc = solver_lib.drot_gl_solve(c.data_ptr(), p.data_ptr(), q.data_ptr(), nr, nc, G, s,
+                                          1e-6, n, -1.0, *ptrs, wptr, nbytes, ctypes.byref(res),
+                                          stream)
+        assert rc == 0
+        torch.cuda.synchronize()
+        out.append(st)
+    for k in out[0]:
+        assert torch.equal(out[0][k], out[1][k]), k
