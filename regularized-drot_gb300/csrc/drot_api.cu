@@ -429,9 +429,9 @@ static int choose_plan(int mode, int nr, int nc, int G, bool aligned4, Plan& pl,
   return make_plan(mode, nr, nc, G, aligned4 ? 4 : 1, false, pl, ctype, ubounds, ch);
 }
 
-// Resident plan of a problem whose tiles fit the chip (up to about 1700 x 1700
-// with FP32 C; faster than the streaming kernel at every size it fits, from
-// 2.6x at 96 x 80 to 2.2x at 1700 x 1700), cached like the
+// Resident plan of a problem whose tiles fit the chip (QR up to about 4100 x
+// 4100, beyond 1900 x 1900 in part; faster than the streaming kernel at every
+// size it takes, from 2.6x at 96 x 80 to 1.27x at 4000 x 4000), cached like the
 // streaming plans (a problem that does not fit is remembered as such).  A
 // pinned launch choice names a shape of the streaming kernel, so it selects
 // that kernel.
@@ -579,14 +579,17 @@ static int read_stats(const void* ws, drot_result* r, cudaStream_t stream) {
 }
 
 // The resident kernel (drot_resident.cuh), where the problem fits it.
-static int run_resident(const SolveArgs& A, const ResidentPlan& pl, drot_result* result) {
+// c, x, ld: the caller's matrices, or the aligned copies.
+static int run_resident(const SolveArgs& A, const ResidentPlan& pl, const void* c, float* x,
+                        long long ld) {
   ResidentParams prm;
   memset(&prm, 0, sizeof(prm));
-  prm.c = A.c; prm.p = A.p; prm.q = A.q; prm.x = A.x;
+  prm.c = c; prm.p = A.p; prm.q = A.q; prm.x = x;
+  prm.ld = ld;
   prm.a = A.a; prm.b = A.b; prm.phi1 = A.phi1; prm.phi2 = A.phi2; prm.alpha = A.alpha;
   prm.nr = A.nr; prm.nc = A.nc;
-  prm.vec_ok = A.nr % 4 == 0 && aligned16(A.x) &&
-               (A.ctype == DROT_C_F32 ? aligned16(A.c) : (((uintptr_t)A.c & 7u) == 0));
+  prm.vec_ok = ld % 4 == 0 && aligned16(x) &&
+               (A.ctype == DROT_C_F32 ? aligned16(c) : (((uintptr_t)c & 7u) == 0));
   prm.s = A.s; prm.kappa = A.kappa; prm.lambda = A.lambda;
   prm.kappa_rcp = (float)(1.0 / (double)A.kappa);
   prm.two_step = div_two_step_exact(prm.kappa, prm.kappa_rcp) ? 1 : 0;
@@ -613,8 +616,31 @@ static int run_resident(const SolveArgs& A, const ResidentPlan& pl, drot_result*
     cudaGetLastError();
     return DROT_ERR_CUDA;
   }
-  if (result) return read_stats(ws, result, A.stream);
   return DROT_OK;
+}
+
+// Copies C and X (unaligned columns) into cpad and xpad, whose columns have
+// ldp rows, the padding zeroed.
+static int copy_in(const SolveArgs& A, void* cpad, float* xpad, long long ldp) {
+  const size_t esz = A.ctype == DROT_C_F32 ? sizeof(float) : 2;
+  const size_t padr = (size_t)(ldp - A.nr);
+  if ((padr && (cudaMemset2DAsync((char*)cpad + A.nr * esz, ldp * esz, 0, padr * esz, A.nc,
+                                  A.stream) != cudaSuccess ||
+                cudaMemset2DAsync(xpad + A.nr, ldp * sizeof(float), 0, padr * sizeof(float),
+                                  A.nc, A.stream) != cudaSuccess)) ||
+      cudaMemcpy2DAsync(cpad, ldp * esz, A.c, A.nr * esz, A.nr * esz, A.nc,
+                        cudaMemcpyDeviceToDevice, A.stream) != cudaSuccess ||
+      cudaMemcpy2DAsync(xpad, ldp * sizeof(float), A.x, A.nr * sizeof(float),
+                        A.nr * sizeof(float), A.nc, cudaMemcpyDeviceToDevice,
+                        A.stream) != cudaSuccess)
+    return DROT_ERR_CUDA;
+  return DROT_OK;
+}
+
+static int copy_out(const SolveArgs& A, const float* xpad, long long ldp) {
+  return cudaMemcpy2DAsync(A.x, A.nr * sizeof(float), xpad, ldp * sizeof(float),
+                           A.nr * sizeof(float), A.nc, cudaMemcpyDeviceToDevice,
+                           A.stream) == cudaSuccess ? DROT_OK : DROT_ERR_CUDA;
 }
 
 static int run_solve(const SolveArgs& A, drot_result* result) {
@@ -623,14 +649,6 @@ static int run_solve(const SolveArgs& A, drot_result* result) {
   if (A.nr <= 0 || A.nc <= 0 || A.max_iters < 0) return DROT_ERR_INVALID_ARG;
   if (((uintptr_t)A.ws & (kAlign - 1)) != 0) return DROT_ERR_WORKSPACE;
   if (A.ctype != DROT_C_F32 && A.ctype != DROT_C_BF16) return DROT_ERR_INVALID_ARG;
-  {
-    // A one-CTA plan has no wait for the stall hook to run out: the streaming
-    // kernel takes the hooked launch.
-    ResidentPlan rp;
-    if (find_resident(A.mode, A.nr, A.nc, A.G, A.ctype, A.bounds, A.stop_every != 0, rp) &&
-        A.ws_bytes >= rp.total && !(rp.grid == 1 && stall_cta_hook() >= 0))
-      return run_resident(A, rp, result);
-  }
   const bool c_aligned = A.ctype == DROT_C_F32 ? aligned16(A.c) : (((uintptr_t)A.c & 7u) == 0);
   const bool aligned4 = A.nr % 4 == 0 && aligned16(A.x) && c_aligned;
   char* ws = (char*)A.ws;
@@ -648,6 +666,25 @@ static int run_solve(const SolveArgs& A, drot_result* result) {
     }
   }
   const long long ld = repack ? ldp : A.nr;
+  {
+    // The resident kernel, where the problem fits it (columns off the vector
+    // boundary only need the copies when part of them stays in global memory).
+    // A one-CTA plan has no wait for the stall hook to run out: the streaming
+    // kernel takes the hooked launch.
+    ResidentPlan rp;
+    if (find_resident(A.mode, A.nr, A.nc, A.G, A.ctype, A.bounds, A.stop_every != 0, rp) &&
+        A.ws_bytes >= rp.total && (!rp.aligned || aligned4 || repack) &&
+        !(rp.grid == 1 && stall_cta_hook() >= 0)) {
+      const bool copy = rp.aligned && repack;
+      int rc = copy ? copy_in(A, cpad, xpad, ldp) : DROT_OK;
+      if (rc == DROT_OK)
+        rc = run_resident(A, rp, copy ? (const void*)cpad : A.c, copy ? xpad : A.x,
+                          copy ? ldp : A.nr);
+      if (rc == DROT_OK && copy) rc = copy_out(A, xpad, ldp);
+      if (rc == DROT_OK && result) rc = read_stats(ws, result, A.stream);
+      return rc;
+    }
+  }
   Plan pl;
   int rc = choose_plan(A.mode, A.nr, A.nc, A.G, aligned4 || repack, pl, A.ctype, A.bounds);
   if (rc != DROT_OK) return rc;
@@ -693,20 +730,7 @@ static int run_solve(const SolveArgs& A, drot_result* result) {
   prm.stall_cta = stall_cta_hook();
 
   if (cudaMemsetAsync(ws, 0, 512, A.stream) != cudaSuccess) return DROT_ERR_CUDA;
-  if (repack) {
-    const size_t esz = A.ctype == DROT_C_F32 ? sizeof(float) : 2;
-    const size_t padr = (size_t)(ldp - A.nr);
-    if ((padr && (cudaMemset2DAsync(cpad + A.nr * esz, ldp * esz, 0, padr * esz, A.nc,
-                                    A.stream) != cudaSuccess ||
-                  cudaMemset2DAsync(xpad + A.nr, ldp * sizeof(float), 0, padr * sizeof(float),
-                                    A.nc, A.stream) != cudaSuccess)) ||
-        cudaMemcpy2DAsync(cpad, ldp * esz, A.c, A.nr * esz, A.nr * esz, A.nc,
-                          cudaMemcpyDeviceToDevice, A.stream) != cudaSuccess ||
-        cudaMemcpy2DAsync(xpad, ldp * sizeof(float), A.x, A.nr * sizeof(float),
-                          A.nr * sizeof(float), A.nc, cudaMemcpyDeviceToDevice,
-                          A.stream) != cudaSuccess)
-      return DROT_ERR_CUDA;
-  }
+  if (repack && copy_in(A, cpad, xpad, ldp) != DROT_OK) return DROT_ERR_CUDA;
   SolveFn fn = kernel_for(A.mode, pl.vec, pl.kv, pl.tma, pl.ctype);
   if (pl.smem > 48 * 1024 &&
       cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -718,10 +742,7 @@ static int run_solve(const SolveArgs& A, drot_result* result) {
     cudaGetLastError();
     return DROT_ERR_CUDA;
   }
-  if (repack && cudaMemcpy2DAsync(A.x, A.nr * sizeof(float), xpad, ldp * sizeof(float),
-                                  A.nr * sizeof(float), A.nc, cudaMemcpyDeviceToDevice,
-                                  A.stream) != cudaSuccess)
-    return DROT_ERR_CUDA;
+  if (repack && copy_out(A, xpad, ldp) != DROT_OK) return DROT_ERR_CUDA;
   if (result) return read_stats(ws, result, A.stream);
   return DROT_OK;
 }

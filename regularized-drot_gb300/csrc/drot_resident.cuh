@@ -6,7 +6,7 @@
 // a CTA owns one tile of X and C in shared memory for the whole solve, and per
 // iteration the CTAs exchange only the tiles' row and column sums.  Measured,
 // us per iteration, streaming -> here: QR 96 x 80 6.9 -> 2.6, 1000 x 1000 9.6
-// -> 3.3, 1500 x 1500 11.3 -> 4.1, 1700 x 1700 12.5 -> 5.6; GL 300 x 200 8.9
+// -> 3.3, 1500 x 1500 11.3 -> 4.1, 1850 x 1850 13.2 -> 5.7; GL 300 x 200 8.9
 // -> 3.3, 1500 x 1000 (2 classes) 12.1 -> 5.8.  Bound by latency: at 1000 x
 // 1000 an iteration of 6300 clocks has two 4-column steps of a warp (1800), the
 // sums over warps and the duals (about 1500), one exchange through L2 (2000)
@@ -24,6 +24,14 @@
 // registers the iteration missed the instruction cache on 43 % of its
 // fetches (2000 x 1500: 700 cycles per column of a warp).
 //
+// Larger QR problems (about 1900 x 1900 to 4100 x 4100) keep the first nsx
+// columns of every warp's X in shared memory and the first nsc of its C; the
+// rest stays in global memory, in L2 at these sizes, and is read where it is
+// used.  us per iteration, streaming -> here: 2000 x 2000 13.4 -> 6.9, 3000 x
+// 3000 18.6 -> 11.3, 4000 x 4000 29.0 -> 22.8, 2600 x 4100 with BF16 C 22.1 ->
+// 15.7.  (Loading a step's global values one step ahead costs the registers
+// of 16 warps a CTA: 3000 x 3000 11.9.)
+//
 // Exchange.  One 64-bit word per row of a band and per column of a chunk, in
 // L2: every CTA adds its partial sum as a fixed-point number (46 fraction
 // bits; integer addition, so the total does not depend on the order) plus a
@@ -39,7 +47,7 @@
 //   Fixed point: a total has an error of at most GC 2^-47, below the rounding
 // of the FP32 duals it updates.  A CTA whose mass would exceed the words'
 // range (or is not finite) adds a poison count to the mass word instead; then
-// every CTA repeats the round with 16 fraction bits fewer (or with counts of
+// every CTA repeats the round with 8 fraction bits fewer (or with counts of
 // infinities and NaNs), so the arithmetic depends on the data of the
 // iteration alone and a solve split into segments gives the same bits.
 //   The squared residual is published as tagged words {value, tag} and read
@@ -59,14 +67,14 @@ constexpr int kResidentMaxWarps = 16;
 // cycles a trip, against 1300 for lines polled by at most 19.
 constexpr int kPairCopies = 16;
 
-// Dynamic shared memory, in order: X slots [cwp][threads] float4 (one or two
-// copies), C slots [cwp][threads], warp row sums [WC][WR * 128], warp
+// Dynamic shared memory, in order: X slots [nsx][threads] float4 (one or two
+// copies), C slots [nsc][threads], warp row sums [WC][WR * 128], warp
 // column sums [WR][ct], group norms [WR][ct] (GL), staged duals of two
 // parities (t1 [rt], t2 [ct]).
-__host__ __device__ constexpr size_t resident_smem_bytes(int threads, int cwp, int wr, int wc,
-                                                         int rt, int ct, size_t csize,
+__host__ __device__ constexpr size_t resident_smem_bytes(int threads, int nsx, int nsc, int wr,
+                                                         int wc, int rt, int ct, size_t csize,
                                                          bool keep_x, bool gl) {
-  return (size_t)cwp * threads * 4 * (csize + sizeof(float) * (keep_x ? 2 : 1)) +
+  return (size_t)threads * 4 * (nsc * csize + nsx * sizeof(float) * (keep_x ? 2 : 1)) +
          sizeof(float) * ((size_t)wc * wr * 128 + (size_t)wr * ct * (gl ? 2 : 1) +
                           2 * ((size_t)rt + ct)) + 64;
 }
@@ -209,9 +217,9 @@ struct LLWait {
 };
 
 // Fixed-point words: 46 fraction bits for rows and columns, 38 for the mass,
-// 16 fewer per level.  In a class round (level < 0) a contribution counts a
+// 8 fewer per level.  In a class round (level < 0) a contribution counts a
 // NaN (bits 40 up) or an infinity (bits 20 up).
-constexpr int kRowBits = 46, kMassBits = 38, kLevelBits = 16;
+constexpr int kRowBits = 46, kMassBits = 38, kLevelBits = 8;
 constexpr unsigned long long kCountOne = 1ull << 56, kPoisonOne = 1ull << 48;
 
 __device__ __forceinline__ float pow2f(int k) {
@@ -303,11 +311,12 @@ drot_resident_kernel(const ResidentParams P) {
   const int lane = tid & 31, warp = tid >> 5;
   const int WR = P.WR, WC = P.WC, rt = P.rt, ct = P.ct;
   const int wc = warp / WR, wr = warp - wc * WR;
-  const int slots = P.cwp * T;
+  const int nsx = P.nsx, nsc = P.nsc;  // slots of X and of C (the rest stay in global memory)
+  const int slots = nsx * T;
   float4* const xa = reinterpret_cast<float4*>(smem_raw) + tid;  // slot j: xa[j * T]
   float4* const xb = xa + (P.keep ? slots : 0);                  // after odd iterations
   CSlot* const cs = reinterpret_cast<CSlot*>(xb - tid + slots) + tid;
-  float* s_row = reinterpret_cast<float*>(cs - tid + slots);
+  float* s_row = reinterpret_cast<float*>(cs - tid + nsc * T);
   float* s_col = s_row + (size_t)WC * WR * 128;
   float* s_nrm = s_col + (size_t)WR * ct;
   float* s_t1 = s_nrm + (MODE == MODE_GL ? (size_t)WR * ct : 0);  // [2][rt]
@@ -335,15 +344,16 @@ drot_resident_kernel(const ResidentParams P) {
   // this warp's columns and this lane's rows (tile coordinates)
   const int wj0 = min(wc * P.cw, w), ncw = min(P.cw, w - wj0);
   const int r0 = wr * 128 + lane * 4;
-  const long long ld = P.nr;
+  const long long ld = P.ld;
   const bool inside = r0 >= head && r0 + 4 <= h;
   const bool whole = P.vec_ok && inside;
+  const bool live_lane = r0 < h;  // slots in global memory: QR, whole vectors of the padded column
   // rows of the tile under every lane of the warp: no row masks
   const bool full = __all_sync(0xffffffffu, inside);
 
   const CT* const cg = reinterpret_cast<const CT*>(P.c);
   // ---- the tile's X and C
-  for (int j = 0; j < P.cwp; ++j) {
+  for (int j = 0; j < nsx; ++j) {
     const long long off = (long long)(c0 + wj0 + j) * ld + base + r0;
     float xv[4] = {0.0f, 0.0f, 0.0f, 0.0f}, cv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if (j >= ncw) {
@@ -365,6 +375,7 @@ drot_resident_kernel(const ResidentParams P) {
         }
     }
     xb[j * T] = make_float4(xv[0], xv[1], xv[2], xv[3]);
+    if (j >= nsc) continue;
     if constexpr (F32C) cs[j * T] = make_float4(cv[0], cv[1], cv[2], cv[3]);
     else cs[j * T] = make_uint2(__float_as_uint(cv[0]), __float_as_uint(cv[1]));
   }
@@ -497,7 +508,7 @@ drot_resident_kernel(const ResidentParams P) {
     // phi = (staged dual + gamma) / n of this lane's rows and of the warp's
     // columns (lane j: column j); -inf beyond the tile.
     f32x2 f01, f23;
-    float f2l;
+    float f2l, f2h = NEG_INF;  // columns below 32, and from 32 on
     {
       float f1[4] = {NEG_INF, NEG_INF, NEG_INF, NEG_INF};
       f2l = NEG_INF;
@@ -506,6 +517,7 @@ drot_resident_kernel(const ResidentParams P) {
         for (int e = 0; e < 4; ++e)
           if (r0 + e >= head && r0 + e < h) f1[e] = __ldg(P.phi1 + base + r0 + e);
         if (lane < ncw) f2l = __ldg(P.phi2 + c0 + wj0 + lane);
+        if (lane + 32 < ncw) f2h = __ldg(P.phi2 + c0 + wj0 + lane + 32);
       } else {
         const float gamma = s_gamma[prv];
         float4 d = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -532,6 +544,8 @@ drot_resident_kernel(const ResidentParams P) {
             if (r0 + e < head || r0 + e >= h) f1[e] = NEG_INF;
         }
         if (lane >= ncw) f2l = NEG_INF;
+        if (lane + 32 < ncw)
+          f2h = div_rn_by(s_t2[prv * ct + wj0 + lane + 32] + gamma, nr_f, P.nr_rcp);
       }
       f01 = x2_pack(f1[0], f1[1]);
       f23 = x2_pack(f1[2], f1[3]);
@@ -543,6 +557,10 @@ drot_resident_kernel(const ResidentParams P) {
       // Even iterations read C and store the folded X^ - sC.  Four columns a
       // step (the slots are padded to whole steps).
       const f32x2 nk = x2_pack(-kappa, -kappa), ky = x2_pack(kappa_rcp, kappa_rcp);
+      // where a step finds X and C: both in shared memory, C in global memory,
+      // both in global memory (the lane's rows of a column are one vector)
+      float* const xg = P.x + (long long)(c0 + wj0) * ld + base + r0;
+      const CT* const ccol = cg + (long long)(c0 + wj0) * ld + base + r0;
       auto update = [&](auto even_tag, auto two_tag) {
         constexpr bool EV = decltype(even_tag)::value, TWO = decltype(two_tag)::value;
         const float4* xi = EV ? xb : xa;
@@ -553,74 +571,109 @@ drot_resident_kernel(const ResidentParams P) {
           const f32x2 m = x2_pack(m0, m1);
           return TWO ? x2_div_rn_two(m, nk, ky) : x2_div_rn_by_fma(m, nk, ky);
         };
+        auto steps = [&](auto place_tag, int j_from, int j_to) {
+          constexpr int PLACE = decltype(place_tag)::value;  // 0, 1, 2 as above
 #pragma unroll 1
-        for (int j0 = 0; j0 < ncw; j0 += 4) {
-          float x[4][4], col[4];
-          f32x2 c01[4], c23[4];
-          unsigned tm[4];
+          for (int j0 = j_from; j0 < j_to; j0 += 4) {
+            float x[4][4], col[4];
+            f32x2 c01[4], c23[4];
+            unsigned tm[4];
+            const float f2w = j0 < 32 ? f2l : f2h;
+            f32x2 x01[4], x23[4];
+            if constexpr (PLACE > 0) {
+              // the global loads of the step first
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            f32x2 t01, t23;
-            x_pairs(xi[u * T], t01, t23);
-            if constexpr (EV) c_pairs(ci[u * T], c01[u], c23[u]);
-            const float f2 = __shfl_sync(0xffffffffu, f2l, j0 + u);
-            const f32x2 f2b = x2_pack(f2, f2);
-            t01 = x2_add(x2_add(t01, f01), f2b);
-            t23 = x2_add(x2_add(t23, f23), f2b);
-            if constexpr (EV) {
-              t01 = x2_fma(ns2, c01[u], t01);
-              t23 = x2_fma(ns2, c23[u], t23);
+              for (int u = 0; u < 4; ++u) {
+                float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                [[maybe_unused]] float w[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                if (live_lane && j0 + u < ncw) {
+                  if constexpr (PLACE == 2) load_vec<4>(xg + (long long)(j0 + u) * ld, v);
+                  if constexpr (EV) load_c_raw<4, CT>(ccol + (long long)(j0 + u) * ld, w);
+                }
+                if constexpr (PLACE == 2) {
+                  x01[u] = x2_pack(v[0], v[1]);
+                  x23[u] = x2_pack(v[2], v[3]);
+                }
+                if constexpr (EV) {
+                  c01[u] = x2_pack(c_at<CT>(w, 0), c_at<CT>(w, 1));
+                  c23[u] = x2_pack(c_at<CT>(w, 2), c_at<CT>(w, 3));
+                }
+              }
             }
-            x2_unpack(t01, x[u][0], x[u][1]);
-            x2_unpack(t23, x[u][2], x[u][3]);
-          }
-          // min of (bits - 1): one instruction per element
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            tm[u] = (unsigned)__float_as_int(x[u][0]) - 1u;
-#pragma unroll
-            for (int e = 1; e < 4; ++e)
-              tm[u] = __viaddmin_u32((unsigned)__float_as_int(x[u][e]), 0xffffffffu, tm[u]);
-          }
-          // a nonzero dividend below 2^-90 anywhere: the IEEE division
-          const bool slow = __any_sync(0xffffffffu,
-                                       min(min(tm[0], tm[1]), min(tm[2], tm[3])) < kDivTinyBitsM1);
-          f32x2 y01[4], y23[4];
-          if (__builtin_expect(slow, 0)) {
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-              y01[u] = x2_pack(div_ieee(fmaxf(x[u][0], 0.0f), kappa),
-                               div_ieee(fmaxf(x[u][1], 0.0f), kappa));
-              y23[u] = x2_pack(div_ieee(fmaxf(x[u][2], 0.0f), kappa),
-                               div_ieee(fmaxf(x[u][3], 0.0f), kappa));
+              if constexpr (PLACE < 2) x_pairs(xi[u * T], x01[u], x23[u]);
+              if constexpr (PLACE == 0 && EV) c_pairs(ci[u * T], c01[u], c23[u]);
+              const float f2 = __shfl_sync(0xffffffffu, f2w, (j0 + u) & 31);
+              const f32x2 f2b = x2_pack(f2, f2);
+              f32x2 t01 = x2_add(x2_add(x01[u], f01), f2b);
+              f32x2 t23 = x2_add(x2_add(x23[u], f23), f2b);
+              if constexpr (EV) {
+                t01 = x2_fma(ns2, c01[u], t01);
+                t23 = x2_fma(ns2, c23[u], t23);
+              }
+              x2_unpack(t01, x[u][0], x[u][1]);
+              x2_unpack(t23, x[u][2], x[u][3]);
             }
-          } else {
+            // min of (bits - 1): one instruction per element
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-              y01[u] = divide(fmaxf(x[u][0], 0.0f), fmaxf(x[u][1], 0.0f));
-              y23[u] = divide(fmaxf(x[u][2], 0.0f), fmaxf(x[u][3], 0.0f));
-            }
-          }
+              tm[u] = (unsigned)__float_as_int(x[u][0]) - 1u;
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            if constexpr (EV) {
-              put_x(xo[u * T], x2_fma(ns2, c01[u], y01[u]), x2_fma(ns2, c23[u], y23[u]));
-              o01 = x2_fma(y01[u], c01[u], o01);
-              o23 = x2_fma(y23[u], c23[u], o23);
+              for (int e = 1; e < 4; ++e)
+                tm[u] = __viaddmin_u32((unsigned)__float_as_int(x[u][e]), 0xffffffffu, tm[u]);
+            }
+            // a nonzero dividend below 2^-90 anywhere: the IEEE division
+            const bool slow = __any_sync(0xffffffffu,
+                                         min(min(tm[0], tm[1]), min(tm[2], tm[3])) < kDivTinyBitsM1);
+            f32x2 y01[4], y23[4];
+            if (__builtin_expect(slow, 0)) {
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                y01[u] = x2_pack(div_ieee(fmaxf(x[u][0], 0.0f), kappa),
+                                 div_ieee(fmaxf(x[u][1], 0.0f), kappa));
+                y23[u] = x2_pack(div_ieee(fmaxf(x[u][2], 0.0f), kappa),
+                                 div_ieee(fmaxf(x[u][3], 0.0f), kappa));
+              }
             } else {
-              put_x(xo[u * T], y01[u], y23[u]);
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                y01[u] = divide(fmaxf(x[u][0], 0.0f), fmaxf(x[u][1], 0.0f));
+                y23[u] = divide(fmaxf(x[u][2], 0.0f), fmaxf(x[u][3], 0.0f));
+              }
             }
-            a01 = x2_add(a01, y01[u]);
-            a23 = x2_add(a23, y23[u]);
-            float u0, u1;
-            x2_unpack(x2_add(y01[u], y23[u]), u0, u1);
-            col[u] = u0 + u1;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              f32x2 n01 = y01[u], n23 = y23[u];
+              if constexpr (EV) {
+                n01 = x2_fma(ns2, c01[u], n01);
+                n23 = x2_fma(ns2, c23[u], n23);
+                o01 = x2_fma(y01[u], c01[u], o01);
+                o23 = x2_fma(y23[u], c23[u], o23);
+              }
+              if constexpr (PLACE < 2) {
+                put_x(xo[u * T], n01, n23);
+              } else if (live_lane && j0 + u < ncw) {
+                put_x(*reinterpret_cast<float4*>(xg + (long long)(j0 + u) * ld), n01, n23);
+              }
+              float u0, u1;
+              x2_unpack(x2_add(y01[u], y23[u]), u0, u1);
+              col[u] = u0 + u1;
+            }
+            // the step's columns first: a quarter of the additions in one chain
+            a01 = x2_add(a01, x2_add(x2_add(y01[0], y01[1]), x2_add(y01[2], y01[3])));
+            a23 = x2_add(a23, x2_add(x2_add(y23[0], y23[1]), x2_add(y23[2], y23[3])));
+            const float cv = fold_columns<4>(col, lane);
+            if (lane < 4 && j0 + lane < ncw) cpart[j0 + lane] = cv;
+            xi += 4 * T;
+            xo += 4 * T;
+            ci += 4 * T;
           }
-          const float cv = fold_columns<4>(col, lane);
-          if (lane < 4 && j0 + lane < ncw) cpart[j0 + lane] = cv;
-          xi += 4 * T;
-          xo += 4 * T;
-          ci += 4 * T;
+          };
+        steps(std::integral_constant<int, 0>(), 0, min(nsc, ncw));
+        if (nsc < ncw) {
+          steps(std::integral_constant<int, 1>(), nsc, min(nsx, ncw));
+          steps(std::integral_constant<int, 2>(), nsx, ncw);
         }
         if constexpr (EV) {
           ob01 = o01;
@@ -909,9 +962,24 @@ drot_resident_kernel(const ResidentParams P) {
   const float4* const xf = last_it >= 0 && (last_it & 1) == 0 ? xa : xb;
   for (int j = 0; j < ncw; ++j) {
     f32x2 x01, x23, c01, c23;
-    x_pairs(xf[j * T], x01, x23);
-    c_pairs(cs[j * T], c01, c23);
     float v[4];
+    float* const xp = P.x + (long long)(c0 + wj0 + j) * ld + base + r0;
+    if (j < nsx) {
+      x_pairs(xf[j * T], x01, x23);
+    } else {
+      if (!unfold || !live_lane) continue;  // in place already
+      load_vec<4>(xp, v);
+      x01 = x2_pack(v[0], v[1]);
+      x23 = x2_pack(v[2], v[3]);
+    }
+    if (j < nsc) {
+      c_pairs(cs[j * T], c01, c23);
+    } else {
+      float w[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      if (live_lane) load_c_raw<4, CT>(cg + (long long)(c0 + wj0 + j) * ld + base + r0, w);
+      c01 = x2_pack(c_at<CT>(w, 0), c_at<CT>(w, 1));
+      c23 = x2_pack(c_at<CT>(w, 2), c_at<CT>(w, 3));
+    }
     if constexpr (MODE == MODE_QR) {
       const f32x2 s2 = x2_pack(s, s);
       if (unfold) {
@@ -931,7 +999,6 @@ drot_resident_kernel(const ResidentParams P) {
       ob01 = x2_fma(x01, c01, ob01);
       ob23 = x2_fma(x23, c23, ob23);
     }
-    float* const xp = P.x + (long long)(c0 + wj0 + j) * ld + base + r0;
     if (whole) {
       store_vec<4>(xp, v);
     } else {

@@ -10,12 +10,13 @@
 namespace drot {
 
 struct ResidentParams {
-  const void* c;  // float or __nv_bfloat16, leading dimension nr
+  const void* c;  // float or __nv_bfloat16
   const float* p;
   const float* q;
   float* x;
   float *a, *b, *phi1, *phi2, *alpha;
   int nr, nc;
+  long long ld;  // leading dimension of X and C
   int vec_ok;  // columns of X and C start on vector boundaries
   float s, kappa, kappa_rcp, nc_rcp, nr_rcp, n_rcp, lambda;  // n_rcp: RN(1 / (nr + nc))
   double res2_stop;
@@ -26,6 +27,7 @@ struct ResidentParams {
   int band_h;     // QR: rows per band
   int rt, ct;     // rows / columns of the largest tile (strides of the buffers)
   int cw, cwp;    // columns per warp, and rounded up to whole steps
+  int nsx, nsc;   // columns per warp with X / C in shared memory (nsc <= nsx <= cwp)
   int two_step;   // QR: the short division sequence is exact for kappa
   int keep;       // two copies of X (see the kernel)
   unsigned long long *rowx, *colx;  // [2][GR][rt], [2][GC][ct] counted fixed-point sums
@@ -41,7 +43,9 @@ struct ResidentParams {
 
 struct ResidentPlan {
   int mode = 0, ctype = 0;
-  int GR = 1, GC = 1, WR = 1, WC = 1, band_h = 0, rt = 0, ct = 0, cw = 0, cwp = 0, keep = 0;
+  int GR = 1, GC = 1, WR = 1, WC = 1, band_h = 0, rt = 0, ct = 0, cw = 0, cwp = 0, nsx = 0, nsc = 0,
+      keep = 0;
+  bool aligned = false;  // needs columns that start on vector boundaries
   int threads = 0, grid = 0;
   size_t smem = 0;
   size_t off_rowx = 0, off_colx = 0, off_massx = 0, off_resx = 0,

@@ -192,3 +192,32 @@ def test_streamed_gl_iterations_recomputed_singly_give_the_same_bits(cuda, solve
         out.append(st)
     for k in out[0]:
         assert torch.equal(out[0][k], out[1][k]), k
+
+
+# part of X and C in global memory: C alone, both, columns off the vector
+# boundary (aligned copies), a ragged last band and chunk, the widest warps
+PARTIAL_SHAPES = [(2000, 2000, torch.float32), (2603, 2501, torch.float32),
+                  (3004, 2998, torch.float32), (2600, 4100, torch.bfloat16),
+                  (4301, 3907, torch.bfloat16), (7000, 900, torch.float32)]
+
+
+@pytest.mark.parametrize("nr,nc,dtype", PARTIAL_SHAPES,
+                         ids=[f"{a}x{b}{'b' if d == torch.bfloat16 else ''}"
+                              for a, b, d in PARTIAL_SHAPES])
+def test_qr_tilings_partly_in_global_memory_match_oracle(cuda, nr, nc, dtype):
+    import reg_drot
+    c, p, q = _problem(nr, nc, nr + nc)
+    c = c.to(dtype)
+    cr = c.float().numpy()
+    for iters in (7, 12):
+        x, info, _ = reg_drot.solve_qr(c.to(cuda), p.to(cuda), q.to(cuda), 2.0, 1e-2, iters, 0.0)
+        o = O.quadratic_drot(cr, p.numpy(), q.numpy(), 2.0, 1e-2, iters, 0.0)
+        assert info["status"] == 0 and info["n_iter"] == iters + 1
+        assert _close(x.cpu(), o["x"])
+        assert abs(info["objective"] - o["objective"]) <= 1e-5 * abs(o["objective"])
+    # a stop: the returned plan is unfolded wherever its columns lie
+    eps = 1.5 * info["residual"]
+    x, info, _ = reg_drot.solve_qr(c.to(cuda), p.to(cuda), q.to(cuda), 2.0, 1e-2, 200, eps)
+    o = O.quadratic_drot(cr, p.numpy(), q.numpy(), 2.0, 1e-2, 200, eps)
+    assert info["converged"] == 1 and info["n_iter"] == o["n_iter"]
+    assert _close(x.cpu(), o["x"])
