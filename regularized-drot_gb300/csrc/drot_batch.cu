@@ -391,7 +391,7 @@ __device__ __forceinline__ void batch_gl_tile_columns(const BatchParams& P, cons
   const CT* const cbase = reinterpret_cast<const CT*>(P.c);
   const int lo = T.lo, hi = T.hi, base = lo & ~3;
   const int nsub = (hi - base + 511) / 512;
-  const int pad = (hi == I.nr && (hi & 3)) ? hi : INT_MAX;  // first padding row, if any
+  const int pad = (I.nr & 3) ? I.nr : INT_MAX;  // first padding row, if any
   const f32x2 ms2 = x2_pack(-I.s, -I.s);
   for (int j = T.c0 + warp; j < T.c1; j += W) {
     const float f2 = __ldcg(P.phi2 + I.col_off + j);
@@ -416,14 +416,14 @@ __device__ __forceinline__ void batch_gl_tile_columns(const BatchParams& P, cons
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
         const int r = base + sb * 512 + v * 128 + lane * VEC;
-        // The caller's padding rows below ld (the last class's vector that
-        // holds row n_rows - 1) may hold any value: their C is zeroed, as y
-        // = 0 there and <C, y> must not see a NaN (a neighbouring class's
-        // rows hold finite costs).
+        // The caller's padding rows below ld (the vector that holds row n_rows
+        // - 1, which short classes share) may hold any value: their C is
+        // zeroed, as y = 0 there and <C, y> must not see a NaN (a neighbouring
+        // class's rows hold finite costs).
         if (r + 4 > pad) {
 #pragma unroll
           for (int e = 0; e < VEC; ++e)
-            if (r + e >= hi) cv[v][e] = 0.0f;
+            if (r + e >= pad) cv[v][e] = 0.0f;
         }
         const float4 f1 = *reinterpret_cast<const float4*>(f1s + (r - base));
         const f32x2 f1p[2] = {x2_pack(f1.x, f1.y), x2_pack(f1.z, f1.w)};
