@@ -599,9 +599,11 @@ static int run_resident(const SolveArgs& A, const ResidentPlan& pl, const void* 
   prm.max_iters = A.max_iters;
   prm.check_all = A.stop_every;
   prm.res2_stop = res2_threshold(A.eps, A.mode == MODE_QR && !A.stop_le);
+  ResidentBounds bounds;
+  memset(&bounds, 0, sizeof(bounds));
   if (A.mode == MODE_GL) {
-    if (A.bounds) std::copy(A.bounds, A.bounds + A.G + 1, prm.gbounds);
-    else group_bounds(A.nr, A.G, prm.gbounds);
+    if (A.bounds) std::copy(A.bounds, A.bounds + A.G + 1, bounds.row);
+    else group_bounds(A.nr, A.G, bounds.row);
   }
   char* const ws = (char*)A.ws;
   prm.stats = (DeviceStats*)ws;
@@ -612,7 +614,7 @@ static int run_resident(const SolveArgs& A, const ResidentPlan& pl, const void* 
   prm.timeout_ns = barrier_timeout_ns();
   prm.stall_cta = stall_cta_hook();
   if (cudaMemsetAsync(ws, 0, pl.total, A.stream) != cudaSuccess) return DROT_ERR_CUDA;
-  if (resident_launch(pl, prm, ws, A.stream) != cudaSuccess) {
+  if (resident_launch(pl, prm, bounds, ws, A.stream) != cudaSuccess) {
     cudaGetLastError();
     return DROT_ERR_CUDA;
   }

@@ -31,6 +31,7 @@
 
 #include "drot_gb300.h"
 #include "drot_kernels.cuh"
+#include "drot_resident.h"
 
 namespace drot {
 
@@ -62,10 +63,7 @@ struct BatchItem {
   int inst, l0, l1, pad;  // lines [l0, l1) of instance inst: row l < nr, column l - nr
 };
 
-struct BatchStat {
-  int n_iter, iters_run, converged, objective_valid;
-  double objective, residual;  // residual: squared on the device, rooted by the host
-};
+typedef BatchRecord BatchStat;
 
 struct BatchParams {
   const void* c;
@@ -1455,6 +1453,12 @@ static inline size_t al(size_t v) { return (v + kAl - 1) / kAl * kAl; }
 struct BatchTuning {
   int fine_cols = 128, finest_cols = 32, item_lines = 1024, finest_item_lines = 64,
       level_quarters = 8, prefetch_distance = 1, tail_quarters = 4;
+  bool operator==(const BatchTuning& o) const {
+    return fine_cols == o.fine_cols && finest_cols == o.finest_cols &&
+           item_lines == o.item_lines && finest_item_lines == o.finest_item_lines &&
+           level_quarters == o.level_quarters && prefetch_distance == o.prefetch_distance &&
+           tail_quarters == o.tail_quarters;
+  }
 };
 static std::mutex g_tuning_mu;
 static BatchTuning g_tuning;
@@ -1486,6 +1490,12 @@ struct BatchPlanImpl {
          off_tobj = 0, off_res = 0, off_obj = 0, off_conv = 0, off_stats = 0, off_act = 0, off_order = 0,
          off_ilvl = 0, off_xn = 0,
          off_yn = 0, total = 0;
+  // resident tiles (drot_resident.cuh), where they are the faster way: records,
+  // class boundaries, CTAs needed and the scheduler's first state (uploaded), then
+  // its state and the exchange words of a launch
+  ResidentBatchPlan res;
+  size_t off_rinst = 0, off_rbounds = 0, off_rneed = 0, off_rfirst = 0, off_rstate = 0,
+         off_rwords = 0;
   bool uploaded_any = false;
 };
 
@@ -1796,6 +1806,22 @@ static int batch_plan_create_impl(int n_inst, const drot_batch_instance* desc, i
     P.grid_pt = occ_pt * sms;
   }
 
+  {
+    std::vector<ResidentInst> ri(n_inst);
+    for (int k = 0; k < n_inst; ++k) {
+      const BatchInst& I = P.inst[k];
+      ResidentInst& r = ri[k];
+      memset(&r, 0, sizeof(r));
+      r.c_off = I.c_off; r.x_off = I.x_off; r.p_off = I.p_off; r.q_off = I.q_off; r.ld = I.ld;
+      r.nr = I.nr; r.nc = I.nc; r.row_off = I.row_off; r.col_off = I.col_off; r.index = k;
+      r.s = I.s; r.kappa = I.kappa; r.kappa_rcp = I.kappa_rcp; r.nc_rcp = I.nc_rcp;
+      r.nr_rcp = I.nr_rcp; r.lambda = I.lambda; r.res2_stop = I.res2_stop;
+      r.n_rcp = (float)(1.0 / (double)(I.nr + I.nc));
+      r.two_step = div_two_step_exact(I.kappa, I.kappa_rcp) ? 1 : 0;
+    }
+    if (P.tune == BatchTuning()) resident_batch_plan(gl ? MODE_GL : MODE_QR, ri, bounds, sms, P.res);
+  }
+
   size_t off = 0;
   P.off_ctrl = off;  off = al(off + 512);
   P.off_inst = off;  off = al(off + sizeof(BatchInst) * n_inst);
@@ -1819,6 +1845,14 @@ static int batch_plan_create_impl(int n_inst, const drot_batch_instance* desc, i
   P.off_ilvl = off;  off = al(off + sizeof(int) * n_inst);
   P.off_xn = off;    off = al(off + sizeof(float) * rows);
   P.off_yn = off;    off = al(off + sizeof(float) * cols);
+  if (P.res.ok) {
+    P.off_rinst = off;   off = al(off + sizeof(ResidentInst) * n_inst);
+    P.off_rbounds = off; off = al(off + sizeof(int) * P.res.bounds.size());
+    P.off_rneed = off;   off = al(off + sizeof(int) * n_inst);
+    P.off_rfirst = off;  off = al(off + sizeof(int) * P.res.state.size());
+    P.off_rstate = off;  off = al(off + sizeof(int) * P.res.state.size());
+    P.off_rwords = off;  off = al(off + sizeof(unsigned long long) * P.res.words);
+  }
   P.total = off;
 
   drot_batch_plan h = new (std::nothrow) drot_batch_plan_s;
@@ -1883,16 +1917,27 @@ int drot_batch_upload(drot_batch_plan plan, void* workspace, size_t workspace_by
       cudaMemcpyAsync(ws + P.off_items, P.items.data(), sizeof(BatchItem) * P.items.size(),
                       cudaMemcpyHostToDevice, st) != cudaSuccess ||
       cudaMemcpyAsync(ws + P.off_order, P.order.data(), sizeof(int) * P.n_inst,
-                      cudaMemcpyHostToDevice, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
+                      cudaMemcpyHostToDevice, st) != cudaSuccess)
     return DROT_ERR_CUDA;
-  return DROT_OK;
+  if (P.res.ok &&
+      (cudaMemcpyAsync(ws + P.off_rneed, P.res.need.data(), sizeof(int) * P.n_inst,
+                       cudaMemcpyHostToDevice, st) != cudaSuccess ||
+       cudaMemcpyAsync(ws + P.off_rfirst, P.res.state.data(), sizeof(int) * P.res.state.size(),
+                       cudaMemcpyHostToDevice, st) != cudaSuccess ||
+       cudaMemcpyAsync(ws + P.off_rinst, P.res.inst.data(), sizeof(ResidentInst) * P.n_inst,
+                       cudaMemcpyHostToDevice, st) != cudaSuccess ||
+       (!P.res.bounds.empty() &&
+        cudaMemcpyAsync(ws + P.off_rbounds, P.res.bounds.data(),
+                        sizeof(int) * P.res.bounds.size(), cudaMemcpyHostToDevice, st) !=
+            cudaSuccess)))
+    return DROT_ERR_CUDA;
+  return cudaStreamSynchronize(st) == cudaSuccess ? DROT_OK : DROT_ERR_CUDA;
 }
 
 // Shared by the cost-matrix and the point-cloud launches: parameter block,
 // control words, warm start, then the cooperative solve kernel `fn`.
 static int batch_launch(const BatchPlanImpl& P, const void* fn, BatchParams& B, void* workspace,
-                        size_t workspace_bytes, int max_iters, cudaStream_t st,
+                        size_t workspace_bytes, int max_iters, cudaStream_t st, int ctype,
                         bool points = false) {
   const int grid = points ? P.grid_pt : P.grid;
   const int threads = points ? P.threads_pt : P.threads;
@@ -1944,6 +1989,41 @@ static int batch_launch(const BatchPlanImpl& P, const void* fn, BatchParams& B, 
   if (cudaMemsetAsync(ws + P.off_ctrl, 0, 512, st) != cudaSuccess) return DROT_ERR_CUDA;
   batch_init_kernel<<<dim3(64, P.n_inst), 256, 0, st>>>(B);
   if (cudaGetLastError() != cudaSuccess) return DROT_ERR_CUDA;
+  // Resident tiles: whole solves of stored costs (the points' cost is made by
+  // the streaming kernel's tiles, the log is of its iterations; the stall hook
+  // needs a CTA that another one waits for).
+  if (P.res.ok && P.res.us < P.res.stream_us[ctype == DROT_C_BF16 ? 1 : 0] && !points && !B.resume && !B.no_stop && B.iter_log_cap == 0 &&
+      (B.stall_cta < 0 || (P.res.first_n > 1 && B.stall_cta < P.res.first_n))) {
+    ResidentBatch R;
+    memset(&R, 0, sizeof(R));
+    R.c = B.c; R.p = B.p; R.q = B.q; R.x = B.x;
+    R.inst = (const ResidentInst*)(ws + P.off_rinst);
+    R.bounds = (const int*)(ws + P.off_rbounds);
+    R.a = B.a; R.b = B.b; R.phi1 = B.phi1; R.phi2 = B.phi2; R.alpha = B.alpha;
+    R.records = B.stats;
+    R.need = (const int*)(ws + P.off_rneed);
+    R.sched = (int*)(ws + P.off_rstate);
+    R.mail = (unsigned*)(R.sched + kSchedWords);
+    R.taken = R.mail + P.res.grid;
+    R.finished = R.taken + P.n_inst;
+    R.free_list = (int*)(R.finished + P.n_inst);
+    R.cta_of = R.free_list + P.res.grid;
+    R.words = (unsigned long long*)(ws + P.off_rwords);
+    R.abort_flag = B.abort_flag;
+    R.n_inst = P.n_inst;
+    R.max_iters = max_iters;
+    R.stall_cta = B.stall_cta;
+    R.timeout_ns = B.timeout_ns;
+    if (cudaMemcpyAsync(R.sched, ws + P.off_rfirst, sizeof(int) * P.res.state.size(),
+                        cudaMemcpyDeviceToDevice, st) != cudaSuccess ||
+        cudaMemsetAsync(R.words, 0, sizeof(unsigned long long) * P.res.words, st) != cudaSuccess)
+      return DROT_ERR_CUDA;
+    if (resident_batch_launch(P.res, P.gl ? MODE_GL : MODE_QR, ctype, R, st) != cudaSuccess) {
+      cudaGetLastError();
+      return DROT_ERR_CUDA;
+    }
+    return DROT_OK;
+  }
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
           cudaSuccess)
@@ -1980,7 +2060,7 @@ int drot_qr_batch_launch(drot_batch_plan plan, const void* c, int c_dtype, const
                        : (gl ? (const void*)batch_solve_kernel<__nv_bfloat16, 0, true>
                              : (const void*)batch_solve_kernel<__nv_bfloat16, 0>);
   return batch_launch(plan->p, fn, B, workspace, workspace_bytes, max_iters,
-                      (cudaStream_t)stream);
+                      (cudaStream_t)stream, c_dtype);
 }
 
 int drot_batch_resume(drot_batch_plan plan, const void* c, int c_dtype, const float* p,
@@ -2004,7 +2084,7 @@ int drot_batch_resume(drot_batch_plan plan, const void* c, int c_dtype, const fl
   const void* fn = c_dtype == DROT_C_F32 ? (const void*)batch_solve_kernel<float, 0, true>
                                          : (const void*)batch_solve_kernel<__nv_bfloat16, 0, true>;
   cudaStream_t st = (cudaStream_t)stream;
-  const int rc = batch_launch(P, fn, B, workspace, workspace_bytes, n_iters, st);
+  const int rc = batch_launch(P, fn, B, workspace, workspace_bytes, n_iters, st, c_dtype);
   if (rc != DROT_OK) return rc;
   // alpha of the last iteration sits in parity slot n_iters & 1: bring it to
   // slot 0, where the next launch reads it.
@@ -2052,7 +2132,7 @@ int drot_qr_batch_launch_points(drot_batch_plan plan, const float* xpts, const f
   if (cudaGetLastError() != cudaSuccess) return DROT_ERR_CUDA;
   const void* fn = dim == 8 ? (const void*)batch_solve_kernel<float, 8>
                             : (const void*)batch_solve_kernel<float, 16>;
-  return batch_launch(P, fn, B, workspace, workspace_bytes, max_iters, st, true);
+  return batch_launch(P, fn, B, workspace, workspace_bytes, max_iters, st, DROT_C_F32, true);
 }
 
 int drot_batch_set_iteration_log(drot_batch_plan plan, unsigned long long* times,

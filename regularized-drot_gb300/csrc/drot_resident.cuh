@@ -70,13 +70,17 @@ constexpr int kPairCopies = 16;
 // Dynamic shared memory, in order: X slots [nsx][threads] float4 (one or two
 // copies), C slots [nsc][threads], warp row sums [WC][WR * 128], warp
 // column sums [WR][ct], group norms [WR][ct] (GL), staged duals of two
-// parities (t1 [rt], t2 [ct]).
+// parities (t1 [rt], t2 [ct]); batches: words seen [2][rt + ct], and GL
+// marginals and former duals [rt + ct].
 __host__ __device__ constexpr size_t resident_smem_bytes(int threads, int nsx, int nsc, int wr,
                                                          int wc, int rt, int ct, size_t csize,
-                                                         bool keep_x, bool gl) {
+                                                         bool keep_x, bool gl, bool batch) {
   return (size_t)threads * 4 * (nsc * csize + nsx * sizeof(float) * (keep_x ? 2 : 1)) +
          sizeof(float) * ((size_t)wc * wr * 128 + (size_t)wr * ct * (gl ? 2 : 1) +
-                          2 * ((size_t)rt + ct)) + 64;
+                          2 * ((size_t)rt + ct)) +
+         (batch ? (2 * sizeof(unsigned long long) + (gl ? 2 * sizeof(float) : 0)) *
+                      ((size_t)rt + ct)
+                : 0) + 64;
 }
 
 // ---- tagged words ---------------------------------------------------------
@@ -300,9 +304,12 @@ __device__ __forceinline__ float fold_columns(float (&m)[NC], int lane) {
 // The kernel
 // ---------------------------------------------------------------------------
 
-template <int MODE, typename CT, int T>
-__global__ void __launch_bounds__(T, 1)
-drot_resident_kernel(const ResidentParams P) {
+// One CTA's part (tile `cta` of G) of one problem's solve.  BATCH: one of a
+// batch's instances (drot_resident_batch_kernel), whose record is a batch
+// record and whose final alpha goes to the slot of its iteration parity.
+template <int MODE, typename CT, int T, bool BATCH>
+__device__ __forceinline__ void resident_solve(const ResidentParams& P, const int* gbounds,
+                                               const int cta, const int G) {
   constexpr bool F32C = std::is_same<CT, float>::value;
   using CSlot = typename std::conditional<F32C, float4, uint2>::type;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -326,15 +333,14 @@ drot_resident_kernel(const ResidentParams P) {
   __shared__ fpair s_r2, s_own;
   __shared__ int s_stop, s_level;
 
-  const int G = gridDim.x;
-  const int br = blockIdx.x / P.GC, bc = blockIdx.x - br * P.GC;
+  const int br = cta / P.GC, bc = cta - br * P.GC;
   int lo, hi;
   if constexpr (MODE == MODE_QR) {
     lo = min(br * P.band_h, P.nr);
     hi = min(lo + P.band_h, P.nr);
   } else {
-    lo = P.gbounds[br];
-    hi = P.gbounds[br + 1];
+    lo = gbounds[br];
+    hi = gbounds[br + 1];
   }
   const int base = lo & ~3;  // the tile's row 0 (16-byte columns: a vector boundary)
   const int c0 = (int)(((long long)P.nc * bc) / P.GC);
@@ -347,9 +353,37 @@ drot_resident_kernel(const ResidentParams P) {
   const long long ld = P.ld;
   const bool inside = r0 >= head && r0 + 4 <= h;
   const bool whole = P.vec_ok && inside;
-  const bool live_lane = r0 < h;  // slots in global memory: QR, whole vectors of the padded column
   // rows of the tile under every lane of the warp: no row masks
   const bool full = __all_sync(0xffffffffu, inside);
+  // Slots in global memory are read as whole vectors (the columns are padded to
+  // them; element by element in the one lane that straddles the edge, an
+  // iteration took twice as long).  Rows of a vector beyond the tile get phi =
+  // -inf, which turns any X there into zero, and in a batch a cost of zero (the
+  // padding is the caller's and may hold anything; a single problem's is a copy
+  // with zeros).  GL stores such a vector element by element: its other rows
+  // are another class's.
+  const bool live_lane = r0 + 4 > head && r0 < h;
+  auto c_inside = [&](const float (&w)[4], f32x2& c01, f32x2& c23) {  // of load_c_raw's w
+    float v[4] = {c_at<CT>(w, 0), c_at<CT>(w, 1), c_at<CT>(w, 2), c_at<CT>(w, 3)};
+    if (BATCH && !full) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] = r0 + e >= head && r0 + e < h ? v[e] : 0.0f;
+    }
+    c01 = x2_pack(v[0], v[1]);
+    c23 = x2_pack(v[2], v[3]);
+  };
+  auto set_x = [&](float* g, f32x2 x01, f32x2 x23) {
+    float v[4];
+    x2_unpack(x01, v[0], v[1]);
+    x2_unpack(x23, v[2], v[3]);
+    if (MODE == MODE_QR || inside) {
+      store_vec<4>(g, v);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (r0 + e >= head && r0 + e < h) g[e] = v[e];
+    }
+  };
 
   const CT* const cg = reinterpret_cast<const CT*>(P.c);
   // ---- the tile's X and C
@@ -407,7 +441,7 @@ drot_resident_kernel(const ResidentParams P) {
   // mass and the residual) owns items t + u * IT; the CTAs of a band hold equal
   // copies of its rows' duals (of a chunk, its columns'), and each counts and
   // writes back its share: rows [sr0, sr1), columns [sc0, sc1).
-  constexpr int NI = 4;
+  constexpr int NI = BATCH && MODE == MODE_GL ? 6 : 4;
   const float most_r = (float)((1ull << 55) / (unsigned)P.GC);
   const float most_c = (float)((1ull << 55) / (unsigned)P.GR);
   const int hr = h - head, n_items = hr + w;
@@ -417,8 +451,17 @@ drot_resident_kernel(const ResidentParams P) {
   const int mass_warp = W - 1, res_warp = W - 2;
   constexpr int IT = T - 64;
   const int item_warps = min(W - 2, (n_items + 31) >> 5);
+  // The words as last read, by round parity.  Batches keep them in shared
+  // memory: two CTAs per SM leave 128 registers a thread and an L1 too small to
+  // hold what is spilled (83 % of the reloads missed it; 16 GL instances of
+  // 256..2048 22.2 -> 19.5 ms with the planner's tiles).
+  unsigned long long seen[2][NI];
+  unsigned long long* const s_seen = reinterpret_cast<unsigned long long*>(s_t2 + 2 * ct);
+  const int seen_n = rt + ct;
+  constexpr bool LEAN = BATCH && MODE == MODE_GL;  // marg and dual_prev there, too
   float dual[NI], dual_prev[NI], marg[NI];
-  unsigned long long seen[2][NI];  // the words as last read, by round parity
+  float* const s_marg = reinterpret_cast<float*>(s_seen + 2 * seen_n);
+  float* const s_prev = s_marg + seen_n;
 #pragma unroll
   for (int u = 0; u < NI; ++u) {
     const int i = tid + u * IT;
@@ -427,8 +470,14 @@ drot_resident_kernel(const ResidentParams P) {
       marg[u] = i < hr ? P.p[lo + i] : P.q[c0 + i - hr];
       dual[u] = i < hr ? P.a[lo + i] : P.b[c0 + i - hr];
     }
-    dual_prev[u] = dual[u];
-    seen[0][u] = seen[1][u] = 0ull;
+    if constexpr (!LEAN) {
+      dual_prev[u] = dual[u];
+    } else if (warp < res_warp && i < n_items) {
+      s_marg[i] = marg[u];
+      s_prev[i] = dual[u];
+    }
+    if constexpr (!BATCH) seen[0][u] = seen[1][u] = 0ull;
+    else if (warp < res_warp && i < n_items) s_seen[i] = s_seen[seen_n + i] = 0ull;
   }
   unsigned long long mass_seen[2] = {0ull, 0ull};
 
@@ -455,8 +504,8 @@ drot_resident_kernel(const ResidentParams P) {
   // Stage times of one CTA in SM clocks, scaled to ns at the end.
   __shared__ long long tacc[4], tp, tp0;
   __shared__ unsigned long long ns0;
-  const bool timer = (int)blockIdx.x == P.timer_cta && tid == 0;
-  if (tid == 0) {
+  const bool timer = !BATCH && cta == P.timer_cta && tid == 0;
+  if (!BATCH && tid == 0) {
     for (int k = 0; k < 4; ++k) tacc[k] = 0;
     tp = tp0 = clock64();
     ns0 = globaltimer_ns();
@@ -471,10 +520,10 @@ drot_resident_kernel(const ResidentParams P) {
   // A warp: the CTA's pair to every copy of a grid-wide array; and the copy
   // this CTA reads.
   auto publish_pair = [&](unsigned long long* to, fpair t, unsigned tag) {
-    ll_store(to + ((size_t)(lane >> 1) * G + blockIdx.x) * 2 + (lane & 1),
+    ll_store(to + ((size_t)(lane >> 1) * G + cta) * 2 + (lane & 1),
              (lane & 1) ? t.lo : t.hi, tag);
   };
-  const size_t my_copy = (size_t)(blockIdx.x % kPairCopies) * G * 2;
+  const size_t my_copy = (size_t)(cta % kPairCopies) * G * 2;
   const size_t pair_words = (size_t)kPairCopies * G * 2;  // of one parity
   // Residual warp: the CTA's squared residual to the grid, and the grid's
   // with the decision.
@@ -502,7 +551,8 @@ drot_resident_kernel(const ResidentParams P) {
   for (; it < P.max_iters; ++it) {
     const int par = it & 1, prv = par ^ 1;
     const bool even = par == 0;
-    const bool mute = it == 0 && (int)blockIdx.x == P.stall_cta;  // test hook
+    const bool mute = it == 0 && cta == P.stall_cta;  // test hook
+    if (BATCH && cta == 0 && tid == 0 && (it & 15) == 0) atomicAdd(P.beat, 1u);
 
     // ------------------------------------------------ X-update of the tile
     // phi = (staged dual + gamma) / n of this lane's rows and of the warp's
@@ -582,22 +632,23 @@ drot_resident_kernel(const ResidentParams P) {
             f32x2 x01[4], x23[4];
             if constexpr (PLACE > 0) {
               // the global loads of the step first
+              float v[4][4], w[4][4];
 #pragma unroll
               for (int u = 0; u < 4; ++u) {
-                float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                [[maybe_unused]] float w[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[u][e] = w[u][e] = 0.0f;
                 if (live_lane && j0 + u < ncw) {
-                  if constexpr (PLACE == 2) load_vec<4>(xg + (long long)(j0 + u) * ld, v);
-                  if constexpr (EV) load_c_raw<4, CT>(ccol + (long long)(j0 + u) * ld, w);
+                  if constexpr (PLACE == 2) load_vec<4>(xg + (long long)(j0 + u) * ld, v[u]);
+                  if constexpr (EV) load_c_raw<4, CT>(ccol + (long long)(j0 + u) * ld, w[u]);
                 }
+              }
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
                 if constexpr (PLACE == 2) {
-                  x01[u] = x2_pack(v[0], v[1]);
-                  x23[u] = x2_pack(v[2], v[3]);
+                  x01[u] = x2_pack(v[u][0], v[u][1]);
+                  x23[u] = x2_pack(v[u][2], v[u][3]);
                 }
-                if constexpr (EV) {
-                  c01[u] = x2_pack(c_at<CT>(w, 0), c_at<CT>(w, 1));
-                  c23[u] = x2_pack(c_at<CT>(w, 2), c_at<CT>(w, 3));
-                }
+                if constexpr (EV) c_inside(w[u], c01[u], c23[u]);
               }
             }
 #pragma unroll
@@ -654,7 +705,7 @@ drot_resident_kernel(const ResidentParams P) {
               if constexpr (PLACE < 2) {
                 put_x(xo[u * T], n01, n23);
               } else if (live_lane && j0 + u < ncw) {
-                put_x(*reinterpret_cast<float4*>(xg + (long long)(j0 + u) * ld), n01, n23);
+                set_x(xg + (long long)(j0 + u) * ld, n01, n23);
               }
               float u0, u1;
               x2_unpack(x2_add(y01[u], y23[u]), u0, u1);
@@ -693,54 +744,92 @@ drot_resident_kernel(const ResidentParams P) {
       const float4* xi = even ? xb : xa;
       float4* xo = even ? xa : xb;
       const CSlot* ci = cs;
+      float* const xg = P.x + (long long)(c0 + wj0) * ld + base + r0;
+      const CT* const ccol = cg + (long long)(c0 + wj0) * ld + base + r0;
+      auto steps = [&](auto place_tag, int j_from, int j_to) {
+        constexpr int PLACE = decltype(place_tag)::value;  // 0, 1, 2 as for QR
 #pragma unroll 1
-      for (int j0 = 0; j0 < ncw; j0 += 8) {
-        f32x2 y01[8], y23[8];
-        float col[8];
+        for (int j0 = j_from; j0 < j_to; j0 += 8) {
+          f32x2 y01[8], y23[8];
+          float col[8];
+          const float f2w = j0 < 32 ? f2l : f2h;
+          [[maybe_unused]] float gv[4][4], gw[4][4];  // four columns in flight
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          f32x2 t01, t23, c01, c23;
-          x_pairs(xi[u * T], t01, t23);
-          c_pairs(ci[u * T], c01, c23);
-          const float f2 = __shfl_sync(0xffffffffu, f2l, j0 + u);
-          const f32x2 f2b = x2_pack(f2, f2);
-          t01 = x2_fma(ns2, c01, x2_add(x2_add(t01, f01), f2b));
-          t23 = x2_fma(ns2, c23, x2_add(x2_add(t23, f23), f2b));
-          float v[4];
-          x2_unpack(t01, v[0], v[1]);
-          x2_unpack(t23, v[2], v[3]);
-          y01[u] = x2_pack(fmaxf(v[0], 0.0f), fmaxf(v[1], 0.0f));
-          y23[u] = x2_pack(fmaxf(v[2], 0.0f), fmaxf(v[3], 0.0f));
-          x2_unpack(x2_fma(y23[u], y23[u], x2_mul(y01[u], y01[u])), v[0], v[1]);
-          col[u] = v[0] + v[1];
-        }
-        const int jl = j0 + (lane & 7);
-        float nsl = fold_columns<8>(col, lane);
-        if (WR > 1) {
-          if (lane < 8 && jl < ncw) s_nrm[wr * ct + wj0 + jl] = nsl;
-          asm volatile("bar.sync %0, %1;" :: "r"(1 + wc), "r"(WR * 32) : "memory");
-          nsl = 0.0f;
-          if (jl < ncw)
-            for (int k = 0; k < WR; ++k) nsl += s_nrm[k * ct + wj0 + jl];
-        }
-        const float scale = gl_shrink(nsl, P.lambda);
+          for (int u = 0; u < 8; ++u) {
+            if constexpr (PLACE > 0) {
+              if ((u & 3) == 0) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const float sc = __shfl_sync(0xffffffffu, scale, u);
-          const f32x2 sc2 = x2_pack(sc, sc);
-          const f32x2 z01 = x2_mul(y01[u], sc2), z23 = x2_mul(y23[u], sc2);
-          put_x(xo[u * T], z01, z23);
-          a01 = x2_add(a01, z01);
-          a23 = x2_add(a23, z23);
-          float u0, u1;
-          x2_unpack(x2_add(z01, z23), u0, u1);
-          col[u] = u0 + u1;
+                for (int k = 0; k < 4; ++k) {
+#pragma unroll
+                  for (int e = 0; e < 4; ++e) gv[k][e] = gw[k][e] = 0.0f;
+                  if (live_lane && j0 + u + k < ncw) {
+                    const long long off = (long long)(j0 + u + k) * ld;
+                    if constexpr (PLACE == 2) load_vec<4>(xg + off, gv[k]);
+                    load_c_raw<4, CT>(ccol + off, gw[k]);
+                  }
+                }
+              }
+            }
+            f32x2 t01, t23, c01, c23;
+            if constexpr (PLACE < 2) {
+              x_pairs(xi[u * T], t01, t23);
+            } else {
+              t01 = x2_pack(gv[u & 3][0], gv[u & 3][1]);
+              t23 = x2_pack(gv[u & 3][2], gv[u & 3][3]);
+            }
+            if constexpr (PLACE == 0) c_pairs(ci[u * T], c01, c23);
+            else c_inside(gw[u & 3], c01, c23);
+            const float f2 = __shfl_sync(0xffffffffu, f2w, (j0 + u) & 31);
+            const f32x2 f2b = x2_pack(f2, f2);
+            t01 = x2_fma(ns2, c01, x2_add(x2_add(t01, f01), f2b));
+            t23 = x2_fma(ns2, c23, x2_add(x2_add(t23, f23), f2b));
+            float v[4];
+            x2_unpack(t01, v[0], v[1]);
+            x2_unpack(t23, v[2], v[3]);
+            y01[u] = x2_pack(fmaxf(v[0], 0.0f), fmaxf(v[1], 0.0f));
+            y23[u] = x2_pack(fmaxf(v[2], 0.0f), fmaxf(v[3], 0.0f));
+            x2_unpack(x2_fma(y23[u], y23[u], x2_mul(y01[u], y01[u])), v[0], v[1]);
+            col[u] = v[0] + v[1];
+          }
+          const int jl = j0 + (lane & 7);
+          float nsl = fold_columns<8>(col, lane);
+          if (WR > 1) {
+            if (lane < 8 && jl < ncw) s_nrm[wr * ct + wj0 + jl] = nsl;
+            asm volatile("bar.sync %0, %1;" :: "r"(1 + wc), "r"(WR * 32) : "memory");
+            nsl = 0.0f;
+            if (jl < ncw)
+              for (int k = 0; k < WR; ++k) nsl += s_nrm[k * ct + wj0 + jl];
+          }
+          const float scale = gl_shrink(nsl, P.lambda);
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const float sc = __shfl_sync(0xffffffffu, scale, u);
+            const f32x2 sc2 = x2_pack(sc, sc);
+            const f32x2 z01 = x2_mul(y01[u], sc2), z23 = x2_mul(y23[u], sc2);
+            if constexpr (PLACE < 2) {
+              put_x(xo[u * T], z01, z23);
+            } else if (live_lane && j0 + u < ncw) {
+              set_x(xg + (long long)(j0 + u) * ld, z01, z23);
+            }
+            a01 = x2_add(a01, z01);
+            a23 = x2_add(a23, z23);
+            float u0, u1;
+            x2_unpack(x2_add(z01, z23), u0, u1);
+            col[u] = u0 + u1;
+          }
+          const float cv = fold_columns<8>(col, lane);
+          if (lane < 8 && jl < ncw) cpart[jl] = cv;
+          xi += 8 * T;
+          xo += 8 * T;
+          ci += 8 * T;
         }
-        const float cv = fold_columns<8>(col, lane);
-        if (lane < 8 && jl < ncw) cpart[jl] = cv;
-        xi += 8 * T;
-        xo += 8 * T;
-        ci += 8 * T;
+      };
+      steps(std::integral_constant<int, 0>(), 0, min(nsc, ncw));
+      if constexpr (BATCH) {
+        if (nsc < ncw) {
+          steps(std::integral_constant<int, 1>(), nsc, min(nsx, ncw));
+          steps(std::integral_constant<int, 2>(), nsx, ncw);
+        }
       }
     }
     // ------------------------------------------------ the tile's sums
@@ -885,7 +974,9 @@ drot_resident_kernel(const ResidentParams P) {
             const int np = row ? P.GC : P.GR;
             if (np > 1) {
               const unsigned long long* const wp = row ? rowp + head + i : colp + i - hr;
-              const unsigned long long old = rp ? seen[1][u] : seen[0][u];
+              unsigned long long old;
+              if constexpr (BATCH) old = s_seen[(rp ? seen_n : 0) + i];
+              else old = rp ? seen[1][u] : seen[0][u];
               unsigned long long got = ll_load(wp);
               wait.until([&]() {
                 if ((unsigned)((got - old) >> 56) == (unsigned)np) return true;
@@ -893,13 +984,15 @@ drot_resident_kernel(const ResidentParams P) {
                 return false;
               });
               const unsigned long long n = (got - old) & (kCountOne - 1ull);
-              if (rp) seen[1][u] = got;
+              if constexpr (BATCH) s_seen[(rp ? seen_n : 0) + i] = got;
+              else if (rp) seen[1][u] = got;
               else seen[0][u] = got;
               tot[u] = level < 0 ? class_value(n)
                                  : from_fixed(n) * pow2f(kLevelBits * level - kRowBits);
             }
-            const float rs = tot[u] - marg[u];
-            dual_prev[u] = dual[u];
+            const float rs = tot[u] - (LEAN ? s_marg[i] : marg[u]);
+            if constexpr (LEAN) s_prev[i] = dual[u];
+            else dual_prev[u] = dual[u];
             dual[u] = dual[u] - rs;
             if (row) s_t1[par * rt + head + i] = dual[u] - rs;
             else s_t2[par * ct + i - hr] = dual[u] - rs;
@@ -924,7 +1017,11 @@ drot_resident_kernel(const ResidentParams P) {
       // The words could not hold this round: again on a coarser scale.
       level = next;
 #pragma unroll
-      for (int u = 0; u < NI; ++u) dual[u] = dual_prev[u];
+      for (int u = 0; u < NI; ++u) {
+        const int i = tid + u * IT;
+        if constexpr (!LEAN) dual[u] = dual_prev[u];
+        else if (warp < res_warp && i < n_items) dual[u] = s_prev[i];
+      }
       __syncthreads();
     }
     ++rd;
@@ -967,7 +1064,9 @@ drot_resident_kernel(const ResidentParams P) {
     if (j < nsx) {
       x_pairs(xf[j * T], x01, x23);
     } else {
-      if (!unfold || !live_lane) continue;  // in place already
+      if ((MODE == MODE_QR && !unfold) || !live_lane) continue;  // in place already
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] = 0.0f;
       load_vec<4>(xp, v);
       x01 = x2_pack(v[0], v[1]);
       x23 = x2_pack(v[2], v[3]);
@@ -977,8 +1076,7 @@ drot_resident_kernel(const ResidentParams P) {
     } else {
       float w[4] = {0.0f, 0.0f, 0.0f, 0.0f};
       if (live_lane) load_c_raw<4, CT>(cg + (long long)(c0 + wj0 + j) * ld + base + r0, w);
-      c01 = x2_pack(c_at<CT>(w, 0), c_at<CT>(w, 1));
-      c23 = x2_pack(c_at<CT>(w, 2), c_at<CT>(w, 3));
+      c_inside(w, c01, c23);
     }
     if constexpr (MODE == MODE_QR) {
       const f32x2 s2 = x2_pack(s, s);
@@ -1013,7 +1111,11 @@ drot_resident_kernel(const ResidentParams P) {
 #pragma unroll
     for (int u = 0; u < NI; ++u) {
       const int i = tid + u * IT;
-      const float d = back ? dual_prev[u] : dual[u];
+      float d = dual[u];
+      if (back) {
+        if constexpr (!LEAN) d = dual_prev[u];
+        else if (i < n_items) d = s_prev[i];
+      }
       if (i >= sr0 && i < sr1) {
         P.a[lo + i] = d;
         P.phi1[lo + i] = div_rn_by(s_t1[fp * rt + head + i] + gamma, nc_f, P.nc_rcp);
@@ -1023,9 +1125,9 @@ drot_resident_kernel(const ResidentParams P) {
       }
     }
   }
-  if ((int)blockIdx.x == 0 && warp == mass_warp && lane == 0) {
-    P.stats->sigma = back ? sigma_prev : sigma;
-    *P.alpha = back ? alpha_prev : alpha;
+  if (cta == 0 && warp == mass_warp && lane == 0) {
+    if constexpr (!BATCH) P.stats->sigma = back ? sigma_prev : sigma;
+    P.alpha[BATCH ? ((last_it + 1) & 1) * P.alpha_stride : 0] = back ? alpha_prev : alpha;
   }
   // objective: CTA pairs to CTA 0
   float u[4];
@@ -1036,8 +1138,8 @@ drot_resident_kernel(const ResidentParams P) {
   const fpair cta_ob = block_sum_fp(ob, s_sum);
   if (warp == 0) {
     if (lane < 2 && G > 1 && !aborted)
-      ll_store(P.objx + 2 * blockIdx.x + lane, lane == 0 ? cta_ob.hi : cta_ob.lo, 1u);
-    if (blockIdx.x == 0) {
+      ll_store(P.objx + 2 * cta + lane, lane == 0 ? cta_ob.hi : cta_ob.lo, 1u);
+    if (cta == 0) {
       fpair t = cta_ob;
       if (G > 1 && !aborted) {
         const PairSum all = ll_pairs(P.objx, G, 1u, P.abort_flag, P.timeout_ns, wait.failed);
@@ -1045,7 +1147,18 @@ drot_resident_kernel(const ResidentParams P) {
         t = all.v;
       }
       const bool late = __any_sync(0xffffffffu, wait.failed);
-      if (lane == 0) {
+      const double r2 = fp_value(last_r2);
+      if (BATCH && lane == 0) {
+        BatchRecord r;
+        r.iters_run = last_it + 1;
+        r.n_iter = MODE == MODE_QR ? (converged ? stop_it : it) + 1 : r.iters_run;
+        r.converged = converged ? 1 : 0;
+        r.objective_valid = obj_valid;
+        r.objective = obj_valid && !aborted ? fp_value(t) : 0.0;
+        r.residual = r2;  // squared; -1 before the first test
+        *P.record = r;
+      }
+      if (!BATCH && lane == 0) {
         DeviceStats* st = P.stats;
         st->iters_run = converged ? stop_it + 1 : it;
         // QR: index of the last iteration + 1, max_iters + 1 without
@@ -1055,14 +1168,224 @@ drot_resident_kernel(const ResidentParams P) {
         st->status = (aborted || late || ld_volatile_i32(P.abort_flag)) ? 3 : 0;
         st->objective_valid = obj_valid;
         st->objective = obj_valid && !aborted ? fp_value(t) : 0.0;
-        const double r2 = fp_value(last_r2);
         st->residual = r2 >= 0.0 ? sqrt(r2) : r2;
       }
     }
   }
-  if (timer) {
+  if (!BATCH && timer) {
     const double scale = (double)(globaltimer_ns() - ns0) / (double)max(1ll, clock64() - tp0);
     for (int k = 0; k < 4; ++k) P.stats->phase_ns[k] = (double)tacc[k] * scale;
+  }
+}
+
+template <int MODE, typename CT, int T>
+__global__ void __launch_bounds__(T, 1)
+drot_resident_kernel(const __grid_constant__ ResidentParams P,
+                     const __grid_constant__ ResidentBounds B) {
+  resident_solve<MODE, CT, T, false>(P, B.row, blockIdx.x, gridDim.x);
+}
+
+// ---------------------------------------------------------------------------
+// Batches
+// ---------------------------------------------------------------------------
+//
+// Many problems in one cooperative launch of two 8-warp CTAs per SM.  Every
+// instance runs on as many CTAs as its tiling has, from its first iteration
+// to its stop, and meets no other instance; two instances share an SM, so one
+// computes while the other waits for its exchange.  The streaming batch kernel
+// takes all instances through every iteration together, so their X and C pass
+// through HBM once per iteration; here only the few that run at a time are
+// read, from L2 where shared memory does not hold them.  us per iteration,
+// streaming -> here: QR 4 instances of 64..512 rows and columns 19 -> 3.5, 8 of
+// 64..2048 30 -> 14, 32 of them (34 M elements) 86 -> 50, 256 (296 M) 501 ->
+// 442; GL 4 of 256..1024 22 -> 7.6, 16 of 256..2048 96 -> 67.  Bound by the
+// arithmetic and the shared-memory pipe of the steps, 0.35 clocks per element
+// and SM for QR (of 0.30 with one tile of 16 warps), and by the CTAs that have
+// nothing to run towards the end (15 % for the 32).
+//
+// CTAs wait in a mailbox for (instance, tile); the last CTA of an instance to
+// finish returns its CTAs to the free list and starts the next instances that
+// fit (in order of work, the first that fits), under a lock; the first ones are
+// in the mail at the launch.  Which CTAs run a tile does not enter any sum.
+// Every wait is bounded: for work, by the time since any instance made progress
+// (the heartbeat that first tiles raise every 16 iterations); for the lock, by
+// the limit of the exchanges.
+
+// Warp 0 with the lock held: starts instances while one fits the free CTAs.
+__device__ __noinline__ void resident_schedule(const ResidentBatch& B) {
+  const int lane = threadIdx.x & 31;
+  int free = __ldcg(B.sched + kSchedFree), head = __ldcg(B.sched + kSchedHead);
+  for (;;) {
+    // the first one not started, then the first from there on that fits
+    while (head < B.n_inst) {
+      const int i = head + lane;
+      const unsigned open =
+          __ballot_sync(0xffffffffu, i < B.n_inst && __ldcg(B.taken + i) == 0u);
+      head += open ? __ffs(open) - 1 : 32;
+      if (open) break;
+    }
+    unsigned fits[kBatchWindow / 32];
+#pragma unroll
+    for (int r = 0; r < kBatchWindow / 32; ++r) {
+      const int i = head + 32 * r + lane;
+      fits[r] = __ballot_sync(0xffffffffu, i < B.n_inst && __ldcg(B.taken + i) == 0u &&
+                                               B.need[i] <= free);
+    }
+    int pick = -1;
+#pragma unroll
+    for (int r = kBatchWindow / 32 - 1; r >= 0; --r)
+      if (fits[r]) pick = head + 32 * r + __ffs(fits[r]) - 1;
+    if (pick < 0) break;
+    const int n = B.need[pick];
+    for (int t = lane; t < n; t += 32) {
+      const int c = __ldcg(B.free_list + free - 1 - t);
+      B.cta_of[B.inst[pick].tile0 + t] = c;
+      asm volatile("st.release.gpu.global.u32 [%0], %1;"
+                   :: "l"(B.mail + c), "r"(((unsigned)(pick + 1) << kMailTileBits) | (unsigned)t)
+                   : "memory");
+    }
+    if (lane == 0) B.taken[pick] = 1u;
+    free -= n;
+    __syncwarp();
+  }
+  if (lane == 0) {
+    B.sched[kSchedFree] = free;
+    B.sched[kSchedHead] = head;
+  }
+  __threadfence();
+  __syncwarp();
+}
+
+// Warp 0 of the last CTA of instance k: its CTAs are free again.
+__device__ __noinline__ void resident_finish(const ResidentBatch& B, const ResidentInst& I) {
+  const int lane = threadIdx.x & 31;
+  int locked = 1;
+  if (lane == 0) {
+    LLWait wait = {B.abort_flag, B.timeout_ns, false};
+    wait.until([&]() {
+      if (atomicCAS(B.sched + kSchedLock, 0, 1) == 0) return true;
+      __nanosleep(100);
+      return false;
+    });
+    locked = !wait.failed;
+  }
+  if (!__shfl_sync(0xffffffffu, locked, 0)) return;
+  __threadfence();
+  const int free = __ldcg(B.sched + kSchedFree);
+  for (int t = lane; t < I.n; t += 32) B.free_list[free + t] = __ldcg(B.cta_of + I.tile0 + t);
+  const int left = __ldcg(B.sched + kSchedLeft) - 1;
+  __syncwarp();
+  if (lane == 0) {
+    B.sched[kSchedFree] = free + I.n;
+    B.sched[kSchedLeft] = left;
+  }
+  __threadfence();
+  __syncwarp();
+  if (left == 0) {
+    for (int c = lane; c < (int)gridDim.x; c += 32)
+      asm volatile("st.release.gpu.global.u32 [%0], %1;" :: "l"(B.mail + c), "r"(kMailEnd)
+                   : "memory");
+  } else {
+    resident_schedule(B);
+  }
+  __threadfence();
+  __syncwarp();
+  if (lane == 0) atomicExch(B.sched + kSchedLock, 0);
+}
+
+// One thread: the next mail of this CTA.
+__device__ __noinline__ unsigned resident_mail(const ResidentBatch& B) {
+  unsigned* const mine = B.mail + blockIdx.x;
+  unsigned long long t0 = globaltimer_ns();
+  int beat = 0;
+  for (unsigned spins = 0;; ++spins) {
+    unsigned m;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(m) : "l"(mine) : "memory");
+    if (m == kMailEnd) return m;
+    if (m != 0u) {
+      // the next one cannot be written before this CTA has finished this tile
+      asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" :: "l"(mine), "r"(0u) : "memory");
+      return m;
+    }
+    if ((spins & 15u) == 15u) {
+      if (ld_volatile_i32(B.abort_flag)) return kMailEnd;
+      const unsigned long long now = globaltimer_ns();
+      const int b = ld_volatile_i32(B.sched + kSchedBeat);
+      if (b != beat) {
+        beat = b;
+        t0 = now;
+      } else if ((long long)(now - t0) > B.timeout_ns) {
+        atomicExch(B.abort_flag, 1);
+        return kMailEnd;
+      }
+    }
+    __nanosleep(200);
+  }
+}
+
+template <int MODE, typename CT>
+__global__ void __launch_bounds__(256, 2)
+drot_resident_batch_kernel(const __grid_constant__ ResidentBatch B) {
+  __shared__ ResidentParams prm;
+  __shared__ unsigned s_mail;
+  const int tid = threadIdx.x, lane = tid & 31, me = blockIdx.x;
+  for (;;) {
+    if (tid == 0) s_mail = resident_mail(B);
+    __syncthreads();
+    const unsigned m = s_mail;
+    if (m == kMailEnd) break;
+    const int k = (int)(m >> kMailTileBits) - 1, tile = (int)(m & ((1u << kMailTileBits) - 1u));
+    const ResidentInst& I = B.inst[k];
+    if (tid == 0) {
+      const ResidentTiling& g = I.tiling;
+      prm.c = reinterpret_cast<const CT*>(B.c) + I.c_off;
+      prm.x = B.x + I.x_off;
+      prm.p = B.p + I.p_off;
+      prm.q = B.q + I.q_off;
+      prm.a = B.a + I.row_off;
+      prm.phi1 = B.phi1 + I.row_off;
+      prm.b = B.b + I.col_off;
+      prm.phi2 = B.phi2 + I.col_off;
+      prm.alpha = B.alpha + I.index;
+      prm.alpha_stride = B.n_inst;
+      prm.nr = I.nr; prm.nc = I.nc; prm.ld = I.ld;
+      prm.vec_ok = 1;  // the plan takes only columns on vector boundaries
+      prm.s = I.s; prm.kappa = I.kappa; prm.kappa_rcp = I.kappa_rcp;
+      prm.nc_rcp = I.nc_rcp; prm.nr_rcp = I.nr_rcp; prm.n_rcp = I.n_rcp;
+      prm.lambda = I.lambda;
+      prm.two_step = I.two_step;
+      prm.res2_stop = I.res2_stop;
+      prm.max_iters = B.max_iters;
+      prm.check_all = 0;
+      prm.GR = g.GR; prm.GC = g.GC; prm.WR = g.WR; prm.WC = g.WC;
+      prm.band_h = g.band_h; prm.rt = g.rt; prm.ct = g.ct;
+      prm.cw = g.cw; prm.cwp = g.cwp; prm.nsx = g.nsx; prm.nsc = g.nsc; prm.keep = g.keep;
+      prm.massx = B.words + I.mass_off;
+      prm.resx = B.words + I.res_off;
+      prm.objx = B.words + I.obj_off;
+      prm.rowx = B.words + I.rowx_off;
+      prm.colx = B.words + I.colx_off;
+      prm.abort_flag = B.abort_flag;
+      prm.odd_flag = reinterpret_cast<int*>(prm.massx + 64);
+      prm.record = B.records + I.index;
+      prm.beat = reinterpret_cast<unsigned*>(B.sched + kSchedBeat);
+      prm.stall_cta = B.stall_cta == me ? tile : -1;  // the test hook names a CTA of the launch
+      prm.timeout_ns = B.timeout_ns;
+    }
+    __syncthreads();
+    resident_solve<MODE, CT, 256, true>(prm, B.bounds + I.bounds_off, tile, I.n);
+    // every thread's writes, then the CTA's count
+    __threadfence();
+    __syncthreads();
+    if (tid < 32) {
+      int last = 0;
+      if (lane == 0) last = atomicAdd(B.finished + k, 1u) + 1u == (unsigned)I.n;
+      if (__shfl_sync(0xffffffffu, last, 0)) {
+        __threadfence();
+        resident_finish(B, I);
+      }
+    }
+    __syncthreads();
   }
 }
 

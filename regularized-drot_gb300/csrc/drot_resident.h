@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include <vector>
+
 #include "drot_kernels.cuh"
 
 namespace drot {
@@ -36,9 +38,70 @@ struct ResidentParams {
   unsigned long long* objx;         // [grid][2]
   int *abort_flag, *odd_flag;       // odd_flag: iteration + 1 of a sum that was not finite
   DeviceStats* stats;
+  struct BatchRecord* record;  // batches: instead of stats
+  int alpha_stride;            // batches: floats between the parity slots of alpha
+  unsigned* beat;              // batches: raised every 16 iterations
   int timer_cta, stall_cta;
   long long timeout_ns;
-  int gbounds[kMaxGroups + 1];
+};
+
+struct ResidentBounds {
+  int row[kMaxGroups + 1];  // GL: row boundaries of the classes
+};
+
+// An instance's result record in a batch's workspace.
+struct BatchRecord {
+  int n_iter, iters_run, converged, objective_valid;
+  double objective, residual;  // residual: squared on the device, rooted by the host
+};
+
+// How an instance of a batch is cut into tiles (fields as in ResidentParams).
+struct ResidentTiling {
+  int GR, GC, WR, WC, band_h, rt, ct, cw, cwp, nsx, nsc, keep;
+};
+
+// One instance of a resident batch launch.
+struct ResidentInst {
+  long long c_off, x_off, p_off, q_off, ld;             // elements of the caller's buffers
+  long long mass_off, res_off, obj_off, rowx_off, colx_off;  // its exchange words
+  int nr, nc, row_off, col_off, index;  // index: its place in the caller's list
+  int n, tile0, bounds_off;             // CTAs, first entry of its tiles, of its boundaries
+  float s, kappa, kappa_rcp, nc_rcp, nr_rcp, n_rcp, lambda;
+  int two_step;
+  double res2_stop;
+  ResidentTiling tiling;
+};
+
+// Mail of a CTA of a batch launch: 0 none, kMailEnd, or (instance + 1) <<
+// kMailTileBits | tile.
+constexpr unsigned kMailEnd = 0xffffffffu;
+constexpr int kMailTileBits = 9;
+constexpr int kBatchWindow = 64;  // instances looked at for one that fits
+// Words of the scheduler's state: lock, free CTAs, first instance not started,
+// instances left to finish, heartbeat.
+enum { kSchedLock = 0, kSchedFree, kSchedHead, kSchedLeft, kSchedBeat, kSchedWords = 64 };
+
+// A batch launch (drot_resident_batch_kernel).
+struct ResidentBatch {
+  const void* c;
+  const float *p, *q;
+  float* x;
+  const ResidentInst* inst;
+  const int* bounds;       // GL: row boundaries, inst.bounds_off
+  float *a, *b, *phi1, *phi2, *alpha;
+  BatchRecord* records;
+  unsigned long long* words;  // zeroed
+  const int* need;         // [n_inst] CTAs of an instance
+  // the scheduler's state, as ResidentBatchPlan::state starts it
+  int* sched;              // [kSchedWords]
+  unsigned* mail;          // [grid]
+  unsigned* taken;         // [n_inst] the instance has been started
+  unsigned* finished;      // [n_inst] CTAs done
+  int* free_list;          // [grid]
+  int* cta_of;             // per instance tile: the CTA that runs it
+  int* abort_flag;
+  int n_inst, max_iters, stall_cta;
+  long long timeout_ns;
 };
 
 struct ResidentPlan {
@@ -59,7 +122,30 @@ bool resident_plan(int mode, int nr, int nc, int G, const int* bounds, int ctype
 
 // Enqueues the solve; ws holds pl.total bytes, zeroed by the caller on the
 // same stream.  prm: problem fields set by the caller, plan fields by this.
-cudaError_t resident_launch(const ResidentPlan& pl, ResidentParams& prm, void* ws,
-                            cudaStream_t stream);
+cudaError_t resident_launch(const ResidentPlan& pl, ResidentParams& prm,
+                            const ResidentBounds& bounds, void* ws, cudaStream_t stream);
+
+// How a batch runs on resident tiles.  inst: in the order the instances start
+// (by decreasing work).
+struct ResidentBatchPlan {
+  bool ok = false;
+  int grid = 0, tiles = 0, first_n = 0;  // first_n: CTAs of the first instance
+  size_t smem = 0, words = 0;            // words: 64-bit exchange words of all instances
+  // Estimated microseconds per iteration here, and of the streaming kernel with
+  // a float and a BF16 cost.
+  double us = 0.0, stream_us[2] = {0.0, 0.0};
+  std::vector<ResidentInst> inst;
+  std::vector<int> bounds, need, state;  // state: the scheduler's at the launch
+};
+
+// Tilings for every instance; ok false where an instance has none or the
+// streaming kernel is the faster one.  inst: problem fields and `index` set;
+// gl_bounds: row boundaries of instance k (GL).
+void resident_batch_plan(int mode, const std::vector<ResidentInst>& inst,
+                         const std::vector<std::vector<int>>& gl_bounds, int sms,
+                         ResidentBatchPlan& pl);
+
+cudaError_t resident_batch_launch(const ResidentBatchPlan& pl, int mode, int ctype,
+                                  const ResidentBatch& b, cudaStream_t stream);
 
 }  // namespace drot
