@@ -27,12 +27,12 @@
 //                       columns of a row) and a byte mask in the layout of C,
 //                       one warp per 32 x 32 block.
 //   adj_pcg_kernel   -- Jacobi-preconditioned CG for a batch of instances in
-//                       one persistent cooperative launch.  Every matvec
-//                       line (a row or a column of an instance) is one warp
-//                       walking the set bits of its mask words and summing
-//                       the search direction staged in shared memory.
+//                       one persistent cooperative launch.  The matvec
+//                       multiplies the bit masks with the digits of the
+//                       search direction on the tensor cores, exactly.
 //                       Two grid barriers per iteration; each instance
 //                       stops on its own relative residual.
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <math.h>
@@ -41,6 +41,8 @@
 #include <string.h>
 
 #include <algorithm>
+#include <queue>
+#include <utility>
 #include <vector>
 
 #include "drot_gb300.h"
@@ -72,7 +74,7 @@ struct AdjParams {
   unsigned char* mask;  // byte mask, layout of C (may be null)
   const float* g;       // upstream gradient dL/dX, layout of C
   double* z;            // solution [a; b]
-  double *r, *d0, *d1, *q, *invdiag, *deg;
+  double *r, *d0, *d1, *q, *invdiag, *deg, *y;  // y = M^-1 r
   unsigned *mcol, *mrow;
   const AdjInst* inst;
   const AdjSeg* seg;
@@ -89,6 +91,7 @@ struct AdjParams {
   int* abort_flag;
   long long timeout_ns;
   int n_inst, n_seg, max_iters;
+  int chunk;            // entries staged as digits at a time, a multiple of 32
   double tol;
 };
 
@@ -135,53 +138,133 @@ __global__ void adj_mask_kernel(const AdjParams A) {
 // batched PCG (FP64 vectors)
 // ---------------------------------------------------------------------------
 
-// Lines per warp step and 32-word blocks per line held in registers: a
-// warp loads the mask words of 4 lines (up to 128 words = 4096 bits each per
-// pass) before it walks any bit, so 16 loads per lane are in flight.
-constexpr int kAdjLines = 4;
-constexpr int kAdjWords = 4;
+// The matvec: for every line, the sum of the direction's entries over the set
+// bits of the line's mask words.  FP64 adds are slow on this part (a warp's add
+// takes 16 clocks of an SM), and adding set bit by set bit cost 110 us per CG
+// iteration at 11 M elements.  Here the sums are exact integer sums on the
+// tensor cores: the entries are written as 72-bit fixed-point numbers on the
+// scale of the instance's largest one (2^-72 of it is far below the rounding
+// of an FP64 sum), cut into 8 digits of 9 bits, and the product of the 0 / 1
+// mask (A: 16 lines x 16 entries) with the digits (B: 16 entries x 8 digits)
+// is an FP16 MMA with FP32 accumulation whose every partial sum is an integer
+// below 2^21 times 2^-24, so nothing is rounded.  The digit sums are added up
+// as 64-bit integers and rounded once, to FP64: at least the accuracy of the
+// FP64 sum, and independent of its order.
+//
+// One mask word (32 entries of a line) is two MMAs.  Their k indices are dealt
+// out so that a lane's operand is one AND: register r (0..3: the two halves of
+// the first MMA's k, then the second's) of thread-in-group t holds bits 4 t + r
+// and 4 t + r + 16, as the FP16 numbers 2^(r - 24); the digits carry 2^-r.
+//
+// us per CG iteration, bits walked -> here: 8 instances of 512..2048 rows and
+// columns with a tenth of the entries on the support 134 -> 17 (0.1 %: 119 ->
+// 17), one of 200 28 -> 12, 64 of 512..4096 715 -> 227 (0.1 %: 241 -> 225).  Of
+// the 8 instances' 32,000 clocks the MMAs take about 6000, the digits 2000, the
+// staged direction 3000, the scalars and sums 12,000 and two grid barriers 8000.
+constexpr int kAdjThreads = 512;
+constexpr int kAdjChunk = 4096;     // entries whose digits are staged at a time, at most
+constexpr int kAdjBlock = 512;      // lines whose sums are held at a time
+constexpr int kAdjDigitBytes = 16;  // of a staged entry
 
-// Sum over the set bits of line l's mask words of the staged vector entries
-// (rows sum the column half, columns the row half); lanes split the words,
-// bits are walked in order, then a shuffle tree.  Deterministic.
-__device__ __forceinline__ void lines_dot(const AdjParams& A, const AdjInst& I, int l0, int l1,
-                                          const double* sv, int lane, double (&out)[kAdjLines]) {
-  double s[kAdjLines];
+__device__ __forceinline__ void mma_mask(float (&c)[4], unsigned a0, unsigned a1, unsigned a2,
+                                         unsigned a3, unsigned b0, unsigned b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 "
+               "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// |v| on the scale of exponent field emax as 72 bits in two halves of 36.
+__device__ __forceinline__ void to_fixed72(double v, int emax, unsigned long long& hi,
+                                           unsigned long long& lo) {
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+  const int e = (int)((bits >> 52) & 0x7ffu);
+  const unsigned long long m = (bits & 0xfffffffffffffull) | 0x10000000000000ull;
+  const int sh = emax - e;
+  const unsigned long long mask = (1ull << 36) - 1ull;
+  hi = sh < 37 ? m >> (17 + sh) : 0ull;
+  lo = (sh <= 19 ? m << (19 - sh) : (sh < 73 ? m >> (sh - 19) : 0ull)) & mask;
+  if (e == 0) hi = lo = 0ull;  // zero (and subnormal)
+}
+
+// Digits of the entries v[0 .. n), n <= kAdjChunk, zero up to whole words, as
+// B operands: word w, lane (digit g, t), register r at [w][4 g + t][r].
+__device__ __forceinline__ void stage_digits(const double* v, int n, int emax, unsigned* B) {
+  const int pairs = (n + 31) / 32 * 16;
+  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
+    const int w = i >> 4, k = i & 15;  // entries 32 w + k and + 16
+    const int j0 = 32 * w + k, j1 = j0 + 16;
+    const double v0 = j0 < n ? v[j0] : 0.0, v1 = j1 < n ? v[j1] : 0.0;
+    unsigned long long h0, l0, h1, l1;
+    to_fixed72(v0, emax, h0, l0);
+    to_fixed72(v1, emax, h1, l1);
+    // +- 2^-r, in both halves
+    const unsigned r = k & 3, one = 0x3c00u - (r << 10);
+    const unsigned sc = (one | (v0 < 0.0 ? 0x8000u : 0u)) |
+                        ((one | (v1 < 0.0 ? 0x8000u : 0u)) << 16);
+    const __half2 scale = *reinterpret_cast<const __half2*>(&sc);
+    unsigned* const to = B + w * 128 + (k >> 2) * 4 + r;
 #pragma unroll
-  for (int u = 0; u < kAdjLines; ++u) s[u] = 0.0;
-  const int nwmax = max(I.nwr, I.nwc);
-  for (int w0 = 0; w0 < nwmax; w0 += 32 * kAdjWords) {
-    unsigned wd[kAdjLines][kAdjWords];
-#pragma unroll
-    for (int u = 0; u < kAdjLines; ++u) {
-      const int l = l0 + u;
-      const bool row = l < I.nr;
-      const int nw = row ? I.nwc : I.nwr;
-      const unsigned* words = row ? A.mrow + I.mr_off + (long long)l * I.nwc
-                                  : A.mcol + I.mc_off + (long long)(l - I.nr) * I.nwr;
-#pragma unroll
-      for (int kk = 0; kk < kAdjWords; ++kk) {
-        const int w = w0 + kk * 32 + lane;
-        wd[u][kk] = (l < l1 && w < nw) ? __ldcg(words + w) : 0u;
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kAdjLines; ++u) {
-      const double* base = (l0 + u < I.nr) ? sv + I.nr : sv;
-#pragma unroll
-      for (int kk = 0; kk < kAdjWords; ++kk) {
-        unsigned m = wd[u][kk];
-        const double* b0 = base + (w0 + kk * 32 + lane) * 32;
-        while (m) {
-          const int b = __ffs(m) - 1;
-          s[u] += b0[b];
-          m &= m - 1u;
-        }
-      }
+    for (int g = 0; g < 8; ++g) {
+      const int s = 27 - 9 * (g & 3);
+      const unsigned d0 = (unsigned)((g < 4 ? h0 : l0) >> s) & 0x1ffu;
+      const unsigned d1 = (unsigned)((g < 4 ? h1 : l1) >> s) & 0x1ffu;
+      // 1024 + digit has the digit as its low bits
+      const unsigned u = 0x64006400u | d0 | (d1 << 16);
+      const __half2 x = __hsub2(*reinterpret_cast<const __half2*>(&u), __half2half2(__ushort_as_half(0x6400)));
+      const __half2 y = __hmul2(x, scale);
+      to[g * 16] = *reinterpret_cast<const unsigned*>(&y);
     }
   }
+}
+
+// Adds the digit sums of `n` lines (n <= kAdjBlock; line l's mask words at
+// words[l * stride + w], w < nw the ones of the staged entries) to acc[l][4]:
+// pairs of digits as integers.  A warp takes 16 lines and a share of the words.
+__device__ __forceinline__ void mask_sums(const unsigned* words, int stride, int n, int nw,
+                                          const unsigned* B, unsigned long long* acc) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int groups = (n + 15) / 16;
+  int ks = 1;
+  while (2 * ks * groups <= W && 8 * ks < nw) ks *= 2;
+  for (int task = warp; task < groups * ks; task += W) {
+    const int grp = task / ks, part = task - grp * ks;
+    const int w0 = nw * part / ks, w1 = nw * (part + 1) / ks;
+    const int la = grp * 16 + g, lb = la + 8;
+    const unsigned* const pa = words + (long long)min(la, n - 1) * stride;
+    const unsigned* const pb = words + (long long)min(lb, n - 1) * stride;
+    float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int w = w0; w < w1; w += 4) {
+      unsigned xa[4], xb[4];
 #pragma unroll
-  for (int u = 0; u < kAdjLines; ++u) out[u] = warp_sum_d(s[u]);
+      for (int u = 0; u < 4; ++u) {
+        xa[u] = w + u < w1 ? __ldg(pa + w + u) >> (4 * t) : 0u;
+        xb[u] = w + u < w1 ? __ldg(pb + w + u) >> (4 * t) : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (w + u >= w1) break;
+        const uint4 b = *reinterpret_cast<const uint4*>(B + (w + u) * 128 + lane * 4);
+        const unsigned a = xa[u], d = xb[u];
+        mma_mask(c, a & 0x00010001u, d & 0x00010001u, a & 0x00020002u, d & 0x00020002u, b.x, b.y);
+        mma_mask(c, a & 0x00040004u, d & 0x00040004u, a & 0x00080008u, d & 0x00080008u, b.z, b.w);
+      }
+    }
+    // c[0], c[1]: digits 2 t, 2 t + 1 of line la; c[2], c[3]: of line lb
+    const long long sa = (long long)((int)(c[0] * 16777216.0f) * 512 + (int)(c[1] * 16777216.0f));
+    const long long sb = (long long)((int)(c[2] * 16777216.0f) * 512 + (int)(c[3] * 16777216.0f));
+    if (la < n) atomicAdd(acc + 4 * la + t, (unsigned long long)sa);
+    if (lb < n) atomicAdd(acc + 4 * lb + t, (unsigned long long)sb);
+  }
+}
+
+// The FP64 value of a line's digit sums.
+__device__ __forceinline__ double mask_sum_value(const unsigned long long* acc, int emax) {
+  double s = (double)(long long)acc[0] * 18014398509481984.0;        // 2^54
+  s = fma((double)(long long)acc[1], 68719476736.0, s);              // 2^36
+  s = fma((double)(long long)acc[2], 262144.0, s) + (double)(long long)acc[3];
+  return emax == 0x7ff ? __longlong_as_double(0x7ff8000000000000ll) : scalbn(s, emax - 1094);
 }
 
 // Degree of line l and the right-hand side entry of the adjoint system: the
@@ -224,22 +307,51 @@ __device__ __forceinline__ void line_degree_rhs(const AdjParams& A, const AdjIns
   rhs = warp_sum_d(s);
 }
 
-// Sum over the segments of an instance of slot[] (fixed order).
+// A warp: sum over the segments of an instance of slot[] (fixed order).
 __device__ __forceinline__ double inst_sum(const double* slot, const AdjInst& I) {
   double s = 0.0;
-  for (int t = 0; t < I.nseg; ++t) s += __ldcg(slot + I.seg0 + t);
-  return s;
+  for (int t = threadIdx.x & 31; t < I.nseg; t += 32) s += __ldcg(slot + I.seg0 + t);
+  return warp_sum_d(s);
+}
+
+// Block sums of one value per line of an n-line segment (thread i has lines i,
+// i + blockDim.x, ...): only the warps that have lines take part.  Thread 0
+// receives them.  Fixed trees.
+template <int N>
+__device__ __forceinline__ void line_sums(double (&v)[N], int n, double (*scratch)[16]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int active = min((int)blockDim.x >> 5, (n + 31) >> 5);
+  if (w < active) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      v[k] = warp_sum_d(v[k]);
+      if (lane == 0) scratch[k][w] = v[k];
+    }
+  }
+  __syncthreads();
+  if (w == 0) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = warp_sum_d(lane < active ? scratch[k][lane] : 0.0);
+  }
 }
 
 // Vectors (r, d, q, z) and the staged direction are FP64: the adjoint system
 // is a graph Laplacian whose support graph is often close to a forest (as
 // many edges as vertices), so it is badly conditioned, and an FP32 CG stops
-// at a solution error far above its residual.  The FP64 work is one add per
-// set mask bit and O(lines) vector updates -- small beside the mask traffic.
-__global__ void __launch_bounds__(256, 2) adj_pcg_kernel(const AdjParams A) {
-  extern __shared__ __align__(16) double sv[];  // the staged direction of one instance
-  __shared__ int s_flag;
+// at a solution error far above its residual.  The FP64 work is O(lines) vector
+// updates; the scalars of an instance are one warp's work each (a division by
+// every warp of the CTA took 3000 clocks).
+__global__ void __launch_bounds__(kAdjThreads, 1) adj_pcg_kernel(const AdjParams A) {
+  extern __shared__ __align__(16) unsigned char adj_smem[];
+  unsigned long long* const acc = reinterpret_cast<unsigned long long*>(adj_smem);  // [kAdjBlock][4]
+  unsigned* const digits = reinterpret_cast<unsigned*>(acc + 4 * kAdjBlock);  // [A.chunk] entries
+  double* const sv = reinterpret_cast<double*>(
+      adj_smem + 32 * kAdjBlock + (size_t)kAdjDigitBytes * A.chunk);  // the staged direction
+  __shared__ int s_flag, s_emax;
   __shared__ double s_red[32 + 1];
+  __shared__ double s_part[2][16];
+  __shared__ double s_step;  // beta, then alpha
+  __shared__ int s_done;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
   const int sg0 = A.cta_seg0[blockIdx.x], sg1 = A.cta_seg0[blockIdx.x + 1];
   const double tol2 = A.tol * A.tol;
@@ -262,6 +374,7 @@ __global__ void __launch_bounds__(256, 2) adj_pcg_kernel(const AdjParams A) {
         A.invdiag[gi] = inv;
         A.deg[gi] = (double)dg;
         A.r[gi] = r0;
+        A.y[gi] = inv * r0;
         A.z[gi] = 0.0;
         ry += r0 * (inv * r0);
         rr += r0 * r0;
@@ -291,60 +404,86 @@ __global__ void __launch_bounds__(256, 2) adj_pcg_kernel(const AdjParams A) {
       const AdjSeg S = A.seg[sg];
       const int k = S.inst;
       const AdjInst I = A.inst[k];
-      const bool done = !(inst_sum(rr_cur, I) > tol2 * inst_sum(A.slot_rr0, I));
-      if (done) {
+      __syncthreads();  // the sums and staged vectors of the segment before are read
+      if (warp == 0) {
+        const double rr = inst_sum(rr_cur, I), rr0 = inst_sum(A.slot_rr0, I);
+        if (lane == 0) s_done = !(rr > tol2 * rr0);
+      } else if (warp == 1 && it > 0) {
+        const double ry = inst_sum(ry_cur, I), ryp = inst_sum(ry_prev, I);
+        if (lane == 0) s_step = ry / ryp;
+      } else if (threadIdx.x == 64) {
+        s_emax = 0;
+      }
+      __syncthreads();
+      if (s_done) {
         if (sg == I.seg0 && threadIdx.x == 0 && !A.conv[k]) {
           A.conv[k] = 1;
           atomicAdd(A.conv_count, 1u);
         }
         continue;
       }
-      const double beta = it == 0 ? 0.0 : inst_sum(ry_cur, I) / inst_sum(ry_prev, I);
+      const double beta = it == 0 ? 0.0 : s_step;
       const int nv = I.nr + I.nc;
-      __syncthreads();
-      // Stage d = M^-1 r + beta d_old for the whole instance: a thread takes
-      // 4 entries and issues their 12 loads before using any.
+      // Stage d = y + beta d_old for the whole instance: a thread takes 4
+      // entries and issues their loads before using any.
+      unsigned top = 0u;  // the largest magnitude's upper word
       for (int t0 = threadIdx.x; t0 < nv; t0 += 4 * blockDim.x) {
-        double iv[4], rv[4], dv0[4];
+        double yv[4], dv0[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int t = t0 + u * blockDim.x;
           const int gi = I.v_off + (t < nv ? t : 0);
-          iv[u] = __ldcg(A.invdiag + gi);
-          rv[u] = __ldcg(A.r + gi);
+          yv[u] = __ldcg(A.y + gi);
           dv0[u] = it == 0 ? 0.0 : __ldcg(dold + gi);
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int t = t0 + u * blockDim.x;
           if (t >= nv) break;
-          const double y = iv[u] * rv[u];
-          const double dv = it == 0 ? y : fma(beta, dv0[u], y);
+          const double dv = it == 0 ? yv[u] : fma(beta, dv0[u], yv[u]);
           sv[t] = dv;
+          top = max(top, (unsigned)__double2hiint(dv) & 0x7fffffffu);
           if (t >= S.l0 && t < S.l1) dcur[I.v_off + t] = dv;
         }
       }
+      top = __reduce_max_sync(0xffffffffu, top);
+      if (lane == 0) atomicMax(&s_emax, (int)(top >> 20));
       __syncthreads();
+      const int emax = s_emax;
       double dq = 0.0;
-      for (int l0 = S.l0 + warp * kAdjLines; l0 < S.l1; l0 += W * kAdjLines) {
-        double s[kAdjLines];
-        lines_dot(A, I, l0, S.l1, sv, lane, s);
-        if (lane == 0) {
-#pragma unroll
-          for (int u = 0; u < kAdjLines; ++u) {
-            const int l = l0 + u;
-            if (l < S.l1) {
-              const int gi = I.v_off + l;
-              const double dl = sv[l];
-              const double qv = fma(__ldcg(A.deg + gi), dl, s[u]);
-              A.q[gi] = qv;
-              dq += dl * qv;
-            }
+      // the segment's rows against the column entries, then its columns
+      // against the row entries
+      for (int side = 0; side < 2; ++side) {
+        const int a0 = side ? max(S.l0, I.nr) : S.l0, a1 = side ? S.l1 : min(S.l1, I.nr);
+        const int K = side ? I.nr : I.nc, stride = side ? I.nwr : I.nwc;
+        const double* const src = side ? sv : sv + I.nr;
+        const unsigned* const words =
+            side ? A.mcol + I.mc_off - (long long)I.nr * I.nwr : A.mrow + I.mr_off;
+        for (int b0 = a0; b0 < a1; b0 += kAdjBlock) {
+          const int n = min(kAdjBlock, a1 - b0);
+          for (int i = threadIdx.x; i < 4 * n; i += blockDim.x) acc[i] = 0ull;
+          for (int k0 = 0; k0 < K; k0 += A.chunk) {
+            const int kn = min(A.chunk, K - k0);
+            // a single chunk stays staged for the blocks that follow
+            if (K > A.chunk || b0 == a0) stage_digits(src + k0, kn, emax, digits);
+            __syncthreads();
+            mask_sums(words + (long long)b0 * stride + (k0 >> 5), stride, n, (kn + 31) >> 5,
+                      digits, acc);
+            __syncthreads();
           }
+          for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const int l = b0 + i, gi = I.v_off + l;
+            const double dl = sv[l];
+            const double qv = fma(__ldcg(A.deg + gi), dl, mask_sum_value(acc + 4 * i, emax));
+            A.q[gi] = qv;
+            dq += dl * qv;
+          }
+          __syncthreads();
         }
       }
-      dq = block_sum_d(dq, s_red);
-      if (threadIdx.x == 0) A.slot_dq[sg] = dq;
+      double sums[1] = {dq};
+      line_sums(sums, min(S.l1 - S.l0, kAdjBlock), s_part);
+      if (threadIdx.x == 0) A.slot_dq[sg] = sums[0];
     }
     if (!grid_barrier(A.bar, A.abort_flag, A.timeout_ns, epoch, &s_flag)) return;
     if (__ldcg(A.conv_count) >= (unsigned)A.n_inst) break;
@@ -355,7 +494,16 @@ __global__ void __launch_bounds__(256, 2) adj_pcg_kernel(const AdjParams A) {
     for (int sg = sg0; sg < sg1; ++sg) {
       const AdjSeg S = A.seg[sg];
       const AdjInst I = A.inst[S.inst];
-      if (!(inst_sum(rr_cur, I) > tol2 * inst_sum(A.slot_rr0, I))) {
+      __syncthreads();
+      if (warp == 0) {
+        const double rr = inst_sum(rr_cur, I), rr0 = inst_sum(A.slot_rr0, I);
+        if (lane == 0) s_done = !(rr > tol2 * rr0);
+      } else if (warp == 1) {
+        const double ry = inst_sum(ry_cur, I), dq = inst_sum(A.slot_dq, I);
+        if (lane == 0) s_step = dq > 0.0 ? ry / dq : 0.0;
+      }
+      __syncthreads();
+      if (s_done) {
         // Converged: carry this segment's r.y and r.r into the next parity's
         // slots, so the instance reads the same (converged) sums on every
         // later iteration and stays stopped.  Without the copy the next
@@ -367,9 +515,8 @@ __global__ void __launch_bounds__(256, 2) adj_pcg_kernel(const AdjParams A) {
         }
         continue;
       }
-      const double dq = inst_sum(A.slot_dq, I);
-      const double alpha = dq > 0.0 ? inst_sum(ry_cur, I) / dq : 0.0;
-      double ry = 0.0, rr = 0.0;
+      const double alpha = s_step;
+      double sums[2] = {0.0, 0.0};  // r.y, r.r
       for (int l = S.l0 + threadIdx.x; l < S.l1; l += blockDim.x) {
         const int gi = I.v_off + l;
         const double zl = fma(alpha, __ldcg(dcur + gi), A.z[gi]);
@@ -377,14 +524,14 @@ __global__ void __launch_bounds__(256, 2) adj_pcg_kernel(const AdjParams A) {
         A.z[gi] = zl;
         A.r[gi] = rl;
         const double yl = __ldcg(A.invdiag + gi) * rl;
-        ry += rl * yl;
-        rr += rl * rl;
+        A.y[gi] = yl;
+        sums[0] += rl * yl;
+        sums[1] += rl * rl;
       }
-      ry = block_sum_d(ry, s_red);
-      rr = block_sum_d(rr, s_red);
+      line_sums(sums, S.l1 - S.l0, s_part);
       if (threadIdx.x == 0) {
-        ry_next[sg] = ry;
-        rr_next[sg] = rr;
+        ry_next[sg] = sums[0];
+        rr_next[sg] = sums[1];
         if (sg == I.seg0) A.iters[S.inst] = it + 1;
       }
     }
@@ -397,9 +544,9 @@ __global__ void __launch_bounds__(256, 2) adj_pcg_kernel(const AdjParams A) {
   for (int sg = sg0; sg < sg1; ++sg) {
     const AdjSeg S = A.seg[sg];
     const AdjInst I = A.inst[S.inst];
-    if (sg == I.seg0 && threadIdx.x == 0) {
-      const double r0 = inst_sum(A.slot_rr0, I);
-      A.relres[S.inst] = r0 > 0.0 ? sqrt(inst_sum(rr_fin, I) / r0) : 0.0;
+    if (sg == I.seg0 && warp == 0) {
+      const double r0 = inst_sum(A.slot_rr0, I), r = inst_sum(rr_fin, I);
+      if (lane == 0) A.relres[S.inst] = r0 > 0.0 ? sqrt(r / r0) : 0.0;
     }
   }
 }
@@ -474,7 +621,7 @@ using namespace drot;
 namespace {
 
 struct AdjLayout {
-  int grid = 0, threads = 256, n_seg = 0, V = 0;
+  int grid = 0, threads = kAdjThreads, n_seg = 0, V = 0, chunk = 0;
   size_t smem = 0;
   std::vector<AdjInst> inst;
   std::vector<AdjSeg> seg;
@@ -490,7 +637,7 @@ int adj_layout(int n_inst, const drot_adjoint_instance* d, AdjLayout& L) {
   if (n_inst <= 0 || n_inst > 65535 || !d) return DROT_ERR_INVALID_ARG;
   L.inst.resize(n_inst);
   long long V = 0, mc = 0, mr = 0, lines = 0;
-  int maxv = 0;
+  int maxv = 0, maxk = 0;
   for (int k = 0; k < n_inst; ++k) {
     const drot_adjoint_instance& a = d[k];
     if (a.n_rows <= 0 || a.n_cols <= 0 || a.ld < a.n_rows || a.c_offset < 0 ||
@@ -518,19 +665,28 @@ int adj_layout(int n_inst, const drot_adjoint_instance* d, AdjLayout& L) {
     V = std::max(V, a.v_offset + a.n_rows + a.n_cols);
     lines += a.n_rows + a.n_cols;
     maxv = std::max(maxv, a.n_rows + a.n_cols);
+    maxk = std::max(maxk, std::max(a.n_rows, a.n_cols));
   }
   if (V > INT32_MAX / 2) return DROT_ERR_UNSUPPORTED;
   L.V = (int)V;
   L.mcol_words = mc;
   L.mrow_words = mr;
-  L.smem = sizeof(double) * (size_t)maxv;
-  if (L.smem > 200 * 1024) return DROT_ERR_UNSUPPORTED;
+  if (sizeof(double) * (size_t)maxv > 200 * 1024) return DROT_ERR_UNSUPPORTED;
 
-  int dev = 0, sms = 0, coop = 0, occ = 0;
+  int dev = 0, sms = 0, coop = 0, occ = 0, optin = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
     return DROT_ERR_CUDA;
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+    return DROT_ERR_CUDA;
+  // The direction, the line sums, and as many of the digits as fit beside them
+  // (all of one side for up to 4096 rows or columns).
+  L.smem = sizeof(double) * (size_t)maxv + 32 * (size_t)kAdjBlock;
+  const long long room = ((long long)optin - 2048 - (long long)L.smem) / kAdjDigitBytes;
+  L.chunk = (int)std::min<long long>(std::min(kAdjChunk, (maxk + 31) & ~31), room & ~31LL);
+  if (L.chunk < 32) return DROT_ERR_UNSUPPORTED;
+  L.smem += (size_t)kAdjDigitBytes * L.chunk;
   if (L.smem > 48 * 1024 &&
       cudaFuncSetAttribute((const void*)adj_pcg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)L.smem) != cudaSuccess)
@@ -542,27 +698,62 @@ int adj_layout(int n_inst, const drot_adjoint_instance* d, AdjLayout& L) {
   const long long want = std::max(1LL, lines / 64);
   L.grid = (int)std::min<long long>((long long)occ * sms, want);
 
-  // Lines [c*lines/G, (c+1)*lines/G) go to CTA c, cut at instance boundaries.
   L.cta_seg0.assign(L.grid + 1, 0);
-  long long base = 0;
-  int k = 0;
-  for (int c = 0; c < L.grid; ++c) {
-    L.cta_seg0[c] = (int)L.seg.size();
-    const long long g0 = lines * c / L.grid, g1 = lines * (c + 1) / L.grid;
-    long long g = g0;
-    while (g < g1) {
-      while (g >= base + L.inst[k].nr + L.inst[k].nc) {
-        base += L.inst[k].nr + L.inst[k].nc;
-        ++k;
+  if (2 * n_inst <= L.grid) {
+    // A CTA takes lines of one instance and one side (a second segment or side
+    // doubles its work, and all wait for it: 8 instances of 512..2048 took 32
+    // us per iteration with the even split below, 17 with this one).  CTA by
+    // CTA to the side whose CTAs take longest, in about clocks: the digits of
+    // the other side's entries, then its lines; whole groups of 16 lines.
+    std::vector<int> ctas(2 * n_inst, 1);
+    auto side = [&](int u) { return u & 1 ? L.inst[u / 2].nc : L.inst[u / 2].nr; };
+    auto cost = [&](int u) {
+      const double k = side(u ^ 1);
+      return 2.0 * k + (double)side(u) / ctas[u] * (k / 32.0 + 15.0);
+    };
+    std::priority_queue<std::pair<double, int>> most;
+    for (int u = 0; u < 2 * n_inst; ++u) most.push({cost(u), u});
+    for (int c = 2 * n_inst; c < L.grid; ++c) {
+      const int u = most.top().second;
+      most.pop();
+      ++ctas[u];
+      most.push({cost(u), u});
+    }
+    int c = 0;
+    for (int u = 0; u < 2 * n_inst; ++u) {
+      const int groups = (side(u) + 15) / 16, l0 = u & 1 ? L.inst[u / 2].nr : 0;
+      for (int j = 0; j < ctas[u]; ++j, ++c) {
+        L.cta_seg0[c] = (int)L.seg.size();
+        AdjSeg S;
+        S.inst = u / 2;
+        S.l0 = l0 + std::min(side(u), (int)((long long)groups * j / ctas[u]) * 16);
+        S.l1 = l0 + std::min(side(u), (int)((long long)groups * (j + 1) / ctas[u]) * 16);
+        S.cta = c;
+        if (S.l1 > S.l0) L.seg.push_back(S);
       }
-      const long long end = std::min(g1, base + L.inst[k].nr + L.inst[k].nc);
-      AdjSeg S;
-      S.inst = k;
-      S.l0 = (int)(g - base);
-      S.l1 = (int)(end - base);
-      S.cta = c;
-      L.seg.push_back(S);
-      g = end;
+    }
+  } else {
+    // Lines [c*lines/G, (c+1)*lines/G) go to CTA c, cut at instance boundaries.
+    long long base = 0;
+    int k = 0;
+    for (int c = 0; c < L.grid; ++c) {
+      L.cta_seg0[c] = (int)L.seg.size();
+      const long long g0 = lines * c / L.grid, g1 = lines * (c + 1) / L.grid;
+      long long g = g0;
+      while (g < g1) {
+        while (g >= base + L.inst[k].nr + L.inst[k].nc) {
+          base += L.inst[k].nr + L.inst[k].nc;
+          ++k;
+        }
+        const long long end = std::min(g1, base + L.inst[k].nr + L.inst[k].nc);
+        AdjSeg S;
+        S.inst = k;
+        S.l0 = (int)(g - base);
+        S.l1 = (int)(end - base);
+        S.cta = c;
+        L.seg.push_back(S);
+        g = end;
+      }
     }
   }
   L.cta_seg0[L.grid] = (int)L.seg.size();
@@ -583,7 +774,7 @@ int adj_layout(int n_inst, const drot_adjoint_instance* d, AdjLayout& L) {
   L.off_cta = off;   off = al256(off + sizeof(int) * (L.grid + 1));
   L.off_mcol = off;  off = al256(off + sizeof(unsigned) * (size_t)mc);
   L.off_mrow = off;  off = al256(off + sizeof(unsigned) * (size_t)mr);
-  L.off_vec = off;   off = al256(off + sizeof(double) * (size_t)V * 6);
+  L.off_vec = off;   off = al256(off + sizeof(double) * (size_t)V * 7);
   L.off_slots = off; off = al256(off + sizeof(double) * (size_t)L.n_seg * 6);
   L.off_iters = off; off = al256(off + sizeof(int) * n_inst);
   L.off_conv = off;  off = al256(off + sizeof(int) * n_inst);
@@ -604,6 +795,8 @@ static void adj_params(const AdjLayout& L, char* ws, AdjParams& A) {
   A.q = vec + 3 * (size_t)L.V;
   A.invdiag = vec + 4 * (size_t)L.V;
   A.deg = vec + 5 * (size_t)L.V;
+  A.y = vec + 6 * (size_t)L.V;
+  A.chunk = L.chunk;
   A.mcol = (unsigned*)(ws + L.off_mcol);
   A.mrow = (unsigned*)(ws + L.off_mrow);
   A.inst = (const AdjInst*)(ws + L.off_inst);
