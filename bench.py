@@ -24,7 +24,7 @@ forward + backward of the differentiable OT loss over one batch:
   plain        the same 64 instances one at a time with the drop-in
                operator's entry point (reg_drot.solve_qr: FP32, forward
                only); batched_over_plain = value / plain.
-  roofline     batch_solve_kernel, the dominant kernel of the step:
+  roofline     drot_resident_batch_kernel, the dominant kernel of the step:
                algorithmic bytes of its launch (12 B per element on the
                iterations that read C, 8 B on the others, 12 B for the final
                unfold) over its measured time, against the measured HBM copy
@@ -786,9 +786,12 @@ def run_gpu(args):
     peak, peak_kind = measured_peak()
     kbytes = solve_bytes(shapes, info)
     ksec = statistics.mean(solve_s)
-    ratio = profile_value("batch_solve_diff16.md", "traffic_over_algorithmic")
+    ratio = profile_value("batch_resident_diff16.md", "traffic_over_algorithmic")
     hbm = hbm_point(dev, flush)
-    roofline = {"bound": "hbm", "kernel": "batch_solve_kernel<float>",
+    # The algorithmic bytes are those of streaming every active instance once
+    # per iteration; on resident tiles few of them reach HBM (traffic).
+    roofline = {"bound": "latency, L2 and shared memory",
+                "kernel": "drot_resident_batch_kernel<QR, float>",
                 "achieved": kbytes / ksec / 1e9, "peak": peak, "unit": "GB/s",
                 "frac": kbytes / ksec / 1e9 / peak, "peak_source": peak_kind,
                 "traffic": ratio * kbytes if ratio else None,

@@ -86,7 +86,9 @@ int drot_gl_group_bounds(int n_rows, int n_groups, int *bounds);
  * points built on them).  Replaces the reference's columns-per-block
  * heuristic (core/drot_qr.hpp:236-239) where a caller -- normally the
  * autotuner reg_drot.tune, which times the candidates on the caller's data
- * -- pins one; zero fields keep the planner's choice.
+ * -- pins one; zero fields keep the planner's choice.  A choice with any
+ * non-zero field selects the streaming kernel; without one the planner takes
+ * resident tiles for problems that fit the chip.
  *   vectors_per_lane  QR: cap 1, 2 or 4 (128-bit vectors per lane: 128-,
  *                     256- or 512-row bands); GL: 1, 2, 4 or 8
  *   warps_per_cta     4..16 (default 8 on the register path, 16 on the ring)

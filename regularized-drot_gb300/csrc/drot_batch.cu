@@ -1992,7 +1992,9 @@ static int batch_launch(const BatchPlanImpl& P, const void* fn, BatchParams& B, 
   // Resident tiles: whole solves of stored costs (the points' cost is made by
   // the streaming kernel's tiles, the log is of its iterations; the stall hook
   // needs a CTA that another one waits for).
-  if (P.res.ok && P.res.us < P.res.stream_us[ctype == DROT_C_BF16 ? 1 : 0] && !points && !B.resume && !B.no_stop && B.iter_log_cap == 0 &&
+  const double stream_us = P.res.stream_us[ctype == DROT_C_BF16 ? 1 : 0] *
+                           (max_iters >= kLongIters ? kLongSolve : 1.0);
+  if (P.res.ok && P.res.us < stream_us && !points && !B.resume && !B.no_stop && B.iter_log_cap == 0 &&
       (B.stall_cta < 0 || (P.res.first_n > 1 && B.stall_cta < P.res.first_n))) {
     ResidentBatch R;
     memset(&R, 0, sizeof(R));

@@ -377,7 +377,7 @@ void resident_batch_plan(int mode, const std::vector<ResidentInst>& inst,
     }
     pl.stream_us[bf16 ? 1 : 0] = us;
   }
-  if (pl.us >= std::max(pl.stream_us[0], pl.stream_us[1])) return;
+  if (pl.us >= kLongSolve * std::max(pl.stream_us[0], pl.stream_us[1])) return;
   pl.grid = grid;
   auto take = [&](size_t words) {  // whole 256-byte units
     const size_t at = pl.words;

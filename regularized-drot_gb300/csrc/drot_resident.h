@@ -125,6 +125,16 @@ bool resident_plan(int mode, int nr, int nc, int G, const int* bounds, int ctype
 cudaError_t resident_launch(const ResidentPlan& pl, ResidentParams& prm,
                             const ResidentBounds& bounds, void* ws, cudaStream_t stream);
 
+// Streaming's estimate holds while every instance is active.  With a budget of
+// kLongIters iterations the instances stop one by one, and streaming ends on a
+// few that leave the GPU idle: resident tiles are taken up to kLongSolve times
+// its estimate there.  Seconds to relative 1e-4, streaming -> resident: 64 QR
+// instances of 512..4096 (377 M elements; with all active resident tiles are 3 %
+// behind) 5.03 -> 4.66, with BF16 C 4.72 -> 4.46; 256 of 64..2048 with BF16 C
+// 2.38 -> 1.87.
+constexpr double kLongSolve = 1.1;
+constexpr int kLongIters = 2000;
+
 // How a batch runs on resident tiles.  inst: in the order the instances start
 // (by decreasing work).
 struct ResidentBatchPlan {
