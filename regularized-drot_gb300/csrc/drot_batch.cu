@@ -1,5 +1,8 @@
 // drot_batch.cu -- batched quadratic-regularised DROT: many independent
 // instances of uneven shape solved in one persistent cooperative launch.
+// Batches whose instances fit resident tiles run a few at a time on those
+// (drot_resident.cuh) where that is faster; the kernel here streams all of them
+// through every iteration together.
 //
 // Work units are tiles (instance, row band, column chunk).  In the fused
 // update every CTA takes tiles from a per-iteration atomic counter until the
