@@ -50,9 +50,11 @@
 // every CTA repeats the round with 8 fraction bits fewer (or with counts of
 // infinities and NaNs), so the arithmetic depends on the data of the
 // iteration alone and a solve split into segments gives the same bits.
-//   The squared residual is published as tagged words {value, tag} and read
-// during the next iteration, whose X-update runs meanwhile into the second
-// copy of X; a converged solve hands back the copy before it.  Where the
+//   The squared residual is published as tagged words {value, tag}, in two
+// slots that take turns (drot_exchange.h: residual_slot, with the order that
+// makes that safe), and read during the next iteration, whose X-update runs
+// meanwhile into the second copy of X; a converged solve hands back the copy
+// before it.  Where the
 // shared memory has no room for two copies the CTAs wait for the residual.
 //   Every poll is bounded by wall time like the streaming kernel's barriers.
 #pragma once
@@ -524,7 +526,10 @@ __device__ __forceinline__ void resident_solve(const ResidentParams& P, const in
              (lane & 1) ? t.lo : t.hi, tag);
   };
   const size_t my_copy = (size_t)(cta % kPairCopies) * G * 2;
-  const size_t pair_words = (size_t)kPairCopies * G * 2;  // of one parity
+  // the words of the residual of iteration k
+  auto res_words = [&](int k) {
+    return P.resx + residual_slot(k, MODE == MODE_GL || P.check_all) * ((size_t)kPairCopies * G * 2);
+  };
   // Residual warp: the CTA's squared residual to the grid, and the grid's
   // with the decision.
   auto publish_res = [&](unsigned long long* to, unsigned tag, bool mute) {
@@ -933,10 +938,10 @@ __device__ __forceinline__ void resident_solve(const ResidentParams& P, const in
       } else if (warp == res_warp) {
         // the residual of the iteration before (once), then this one's
         if (P.keep && pend >= 0 && !decided)
-          decide(P.resx + (pend & 1) * pair_words, pend_tag);
+          decide(res_words(pend), pend_tag);
         if (check) {
           asm volatile("bar.sync 15, %0;" :: "r"((item_warps + 1) * 32) : "memory");
-          publish_res(P.resx + par * pair_words, rd + 1u, mute);
+          publish_res(res_words(it), rd + 1u, mute);
         }
       } else if (warp < item_warps) {
         unsigned long long* const rowp = P.rowx + (size_t)(rp * P.GR + br) * rt;
@@ -1033,7 +1038,7 @@ __device__ __forceinline__ void resident_solve(const ResidentParams& P, const in
       pend = it;
       pend_tag = rd;
       if (!P.keep) {
-        if (warp == res_warp) decide(P.resx + par * pair_words, pend_tag);
+        if (warp == res_warp) decide(res_words(it), pend_tag);
         if (__syncthreads_or(wait.failed ? 1 : 0)) { aborted = true; break; }
         last_r2 = s_r2;
         if (s_stop) { stop_it = it; break; }
@@ -1043,7 +1048,7 @@ __device__ __forceinline__ void resident_solve(const ResidentParams& P, const in
   }
   if (P.keep && stop_it < 0 && !aborted && pend >= 0) {
     // max_iters ended on an iteration that is checked: its residual is still out
-    if (warp == res_warp) decide(P.resx + (pend & 1) * pair_words, pend_tag);
+    if (warp == res_warp) decide(res_words(pend), pend_tag);
     if (__syncthreads_or(wait.failed ? 1 : 0)) aborted = true;
     last_r2 = s_r2;
     if (!aborted && s_stop) stop_it = pend;

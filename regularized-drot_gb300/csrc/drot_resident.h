@@ -7,6 +7,7 @@
 
 #include <vector>
 
+#include "drot_exchange.h"
 #include "drot_kernels.cuh"
 
 namespace drot {
@@ -34,7 +35,7 @@ struct ResidentParams {
   int keep;       // two copies of X (see the kernel)
   unsigned long long *rowx, *colx;  // [2][GR][rt], [2][GC][ct] counted fixed-point sums
   unsigned long long* massx;        // [2] of them, 256 bytes apart
-  unsigned long long* resx;         // [2][kPairCopies][grid][2] tagged (hi, lo)
+  unsigned long long* resx;         // [2 slots][kPairCopies][grid][2] tagged (hi, lo)
   unsigned long long* objx;         // [grid][2]
   int *abort_flag, *odd_flag;       // odd_flag: iteration + 1 of a sum that was not finite
   DeviceStats* stats;
