@@ -47,6 +47,7 @@
 
 #include "drot_gb300.h"
 #include "drot_kernels.cuh"
+#include "drot_launch.h"
 
 namespace drot {
 
@@ -687,10 +688,7 @@ int adj_layout(int n_inst, const drot_adjoint_instance* d, AdjLayout& L) {
   L.chunk = (int)std::min<long long>(std::min(kAdjChunk, (maxk + 31) & ~31), room & ~31LL);
   if (L.chunk < 32) return DROT_ERR_UNSUPPORTED;
   L.smem += (size_t)kAdjDigitBytes * L.chunk;
-  if (L.smem > 48 * 1024 &&
-      cudaFuncSetAttribute((const void*)adj_pcg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)L.smem) != cudaSuccess)
-    return DROT_ERR_CUDA;
+  if (allow_shared_memory((const void*)adj_pcg_kernel) != cudaSuccess) return DROT_ERR_CUDA;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void*)adj_pcg_kernel, L.threads,
                                                     L.smem) != cudaSuccess || occ <= 0)
     return DROT_ERR_CUDA;

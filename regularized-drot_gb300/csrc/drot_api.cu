@@ -18,6 +18,7 @@
 
 #include "drot_gb300.h"
 #include "drot_kernels.cuh"
+#include "drot_launch.h"
 #include "drot_resident.h"
 
 namespace drot {
@@ -274,9 +275,7 @@ static int make_plan_uncached(int mode, int nr, int nc, int G, int vec, bool tma
     pl.threads = 32 * warps;
     pl.smem = solve_smem_bytes(warps, pl.wt, S, pl.ns, tma);
     if (pl.smem > budget) return DROT_ERR_UNSUPPORTED;
-    if (pl.smem > 48 * 1024 &&
-        cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)pl.smem) != cudaSuccess)
+    if (pl.smem > 48 * 1024 && allow_shared_memory((const void*)fn) != cudaSuccess)
       return DROT_ERR_CUDA;
     const int occ = occupancy(fn, pl.threads, pl.smem);
     if (occ <= 0) return DROT_ERR_CUDA;
@@ -317,9 +316,7 @@ static int make_plan_uncached(int mode, int nr, int nc, int G, int vec, bool tma
   pl.p2_cap_r = pl.p2_cap_c = 0;
   if ((size_t)p2f * sizeof(float) <= 48 * 1024 && smem2 <= budget) {
     bool ok = true;
-    if (smem2 > 48 * 1024)
-      ok = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem2) == cudaSuccess;
+    if (smem2 > 48 * 1024) ok = allow_shared_memory((const void*)fn) == cudaSuccess;
     if (ok && occupancy(fn, pl.threads, smem2) * dev.sms >= pl.grid) {
       pl.p2_smem = 1;
       pl.p2_cap_r = capr;
@@ -734,9 +731,7 @@ static int run_solve(const SolveArgs& A, drot_result* result) {
   if (cudaMemsetAsync(ws, 0, 512, A.stream) != cudaSuccess) return DROT_ERR_CUDA;
   if (repack && copy_in(A, cpad, xpad, ldp) != DROT_OK) return DROT_ERR_CUDA;
   SolveFn fn = kernel_for(A.mode, pl.vec, pl.kv, pl.tma, pl.ctype);
-  if (pl.smem > 48 * 1024 &&
-      cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)pl.smem) != cudaSuccess)
+  if (pl.smem > 48 * 1024 && allow_shared_memory((const void*)fn) != cudaSuccess)
     return DROT_ERR_CUDA;
   void* args[] = {(void*)&prm};
   if (cudaLaunchCooperativeKernel((const void*)fn, dim3(pl.grid), dim3(pl.threads), args,

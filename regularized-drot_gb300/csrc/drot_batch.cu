@@ -34,6 +34,7 @@
 
 #include "drot_gb300.h"
 #include "drot_kernels.cuh"
+#include "drot_launch.h"
 #include "drot_resident.h"
 
 namespace drot {
@@ -1786,10 +1787,7 @@ static int batch_plan_create_impl(int n_inst, const drot_batch_instance* desc, i
   auto occupancy = [&](const Variant* v, int n, int threads, int& occ) -> bool {
     occ = 1 << 30;
     for (int i = 0; i < n; ++i) {
-      if (v[i].smem > 48 * 1024 &&
-          cudaFuncSetAttribute(v[i].fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)v[i].smem) != cudaSuccess)
-        return false;
+      if (v[i].smem > 48 * 1024 && allow_shared_memory(v[i].fn) != cudaSuccess) return false;
       int o = 0;
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, v[i].fn, threads, v[i].smem) !=
           cudaSuccess)
@@ -2029,10 +2027,7 @@ static int batch_launch(const BatchPlanImpl& P, const void* fn, BatchParams& B, 
     }
     return DROT_OK;
   }
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-          cudaSuccess)
-    return DROT_ERR_CUDA;
+  if (smem > 48 * 1024 && allow_shared_memory(fn) != cudaSuccess) return DROT_ERR_CUDA;
   void* args[] = {(void*)&B};
   if (cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, smem, st) !=
       cudaSuccess) {

@@ -9,6 +9,7 @@
 #include <utility>
 
 #include "drot_gb300.h"
+#include "drot_launch.h"
 
 namespace drot {
 
@@ -127,8 +128,7 @@ bool resident_plan(int mode, int nr, int nc, int G, const int* bounds, int ctype
   if (!found) return false;
   const ResidentFn fn = resident_fn(mode, ctype, best.threads);
   int occ = 0;
-  if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)best.smem) != cudaSuccess ||
+  if (allow_shared_memory((const void*)fn) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void*)fn, best.threads,
                                                     best.smem) != cudaSuccess ||
       occ < 1) {
@@ -160,9 +160,7 @@ cudaError_t resident_launch(const ResidentPlan& pl, ResidentParams& prm,
   prm.rowx = at(pl.off_rowx); prm.colx = at(pl.off_colx);
   prm.massx = at(pl.off_massx); prm.resx = at(pl.off_resx); prm.objx = at(pl.off_objx);
   const ResidentFn fn = resident_fn(pl.mode, pl.ctype, pl.threads);
-  cudaError_t rc = cudaFuncSetAttribute((const void*)fn,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)pl.smem);
+  const cudaError_t rc = allow_shared_memory((const void*)fn);
   if (rc != cudaSuccess) return rc;
   void* args[] = {(void*)&prm, (void*)&bounds};
   return cudaLaunchCooperativeKernel((const void*)fn, dim3(pl.grid), dim3(pl.threads), args,
@@ -429,8 +427,7 @@ void resident_batch_plan(int mode, const std::vector<ResidentInst>& inst,
   for (int ctype : {DROT_C_F32, DROT_C_BF16}) {
     const void* fn = (const void*)resident_batch_fn(mode, ctype);
     int occ = 0;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem) !=
-            cudaSuccess ||
+    if (allow_shared_memory(fn) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 256, pl.smem) != cudaSuccess ||
         occ < 2) {
       cudaGetLastError();
@@ -443,8 +440,7 @@ void resident_batch_plan(int mode, const std::vector<ResidentInst>& inst,
 cudaError_t resident_batch_launch(const ResidentBatchPlan& pl, int mode, int ctype,
                                   const ResidentBatch& b, cudaStream_t stream) {
   const void* fn = (const void*)resident_batch_fn(mode, ctype);
-  const cudaError_t rc =
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
+  const cudaError_t rc = allow_shared_memory(fn);
   if (rc != cudaSuccess) return rc;
   void* args[] = {(void*)&b};
   return cudaLaunchCooperativeKernel(fn, dim3(pl.grid), dim3(256), args, pl.smem, stream);
