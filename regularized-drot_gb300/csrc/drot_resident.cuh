@@ -1015,10 +1015,14 @@ __device__ __forceinline__ void resident_solve(const ResidentParams& P, const in
       if (P.keep && pend >= 0 && !decided) {
         last_r2 = s_r2;
         decided = true;
-        if (s_stop) { stop_it = pend; break; }
       }
       const int next = s_level;
-      if (next == 0) break;
+      if (next == 0) {
+        // a stop ends the loop after a round that the words held, which leaves
+        // alpha and the duals one iteration ahead together
+        if (decided && s_stop) stop_it = pend;
+        break;
+      }
       // The words could not hold this round: again on a coarser scale.
       level = next;
 #pragma unroll
