@@ -13,7 +13,11 @@
 #include <string.h>
 
 #include <algorithm>
+#include <iterator>
+#include <map>
 #include <mutex>
+#include <tuple>
+#include <utility>
 #include <vector>
 
 #include "drot_gb300.h"
@@ -348,34 +352,64 @@ struct PlanKey {
   int dev, mode, nr, nc, G, vec, tma, ctype;
   std::vector<int> ubounds;  // caller's GL group boundaries (empty: the reference's)
   LaunchChoice ch;
-  bool operator==(const PlanKey& o) const {
-    return dev == o.dev && mode == o.mode && nr == o.nr && nc == o.nc && G == o.G &&
-           vec == o.vec && tma == o.tma && ctype == o.ctype && ubounds == o.ubounds && ch == o.ch;
+  bool check_all;            // resident plans
+  bool operator<(const PlanKey& o) const {
+    return std::tie(dev, mode, nr, nc, G, vec, tma, ctype, check_all, ch.kv, ch.warps, ch.tma,
+                    ch.ctas, ubounds) <
+           std::tie(o.dev, o.mode, o.nr, o.nc, o.G, o.vec, o.tma, o.ctype, o.check_all, o.ch.kv,
+                    o.ch.warps, o.ch.tma, o.ch.ctas, o.ubounds);
   }
 };
 
-static std::mutex g_plan_mu;
-static std::vector<std::pair<PlanKey, Plan>> g_plans;
+// A bounded map; when it is full, the half that was not used for longest goes.
+// 4096 entries (about 1 MB) hold the plans of some 1300 shapes.  With 64, first
+// in first out, a program that took 30 shapes in turn planned anew on every call
+// (199 us per call of a 4-iteration solve, against 92 with 8 shapes).
+template <typename V>
+class PlanCache {
+ public:
+  bool find(const PlanKey& key, V& out) {
+    std::lock_guard<std::mutex> lk(mu_);
+    auto it = map_.find(key);
+    if (it == map_.end()) return false;
+    it->second.second = ++clock_;
+    out = it->second.first;
+    return true;
+  }
+  void put(const PlanKey& key, const V& v) {
+    std::lock_guard<std::mutex> lk(mu_);
+    if (map_.size() >= kMost) {
+      std::vector<unsigned long long> used;
+      for (auto& e : map_) used.push_back(e.second.second);
+      std::nth_element(used.begin(), used.begin() + kMost / 2, used.end());
+      const unsigned long long from = used[kMost / 2];
+      for (auto it = map_.begin(); it != map_.end();)
+        it = it->second.second < from ? map_.erase(it) : std::next(it);
+    }
+    map_[key] = {v, ++clock_};
+  }
+
+ private:
+  static constexpr size_t kMost = 4096;
+  std::mutex mu_;
+  std::map<PlanKey, std::pair<V, unsigned long long>> map_;  // plan, last use
+  unsigned long long clock_ = 0;
+};
+
+static PlanCache<Plan> g_plans;
 
 static int make_plan(int mode, int nr, int nc, int G, int vec, bool tma, Plan& pl,
                      int ctype = DROT_C_F32, const int* ubounds = nullptr,
                      const LaunchChoice& ch = LaunchChoice()) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return DROT_ERR_CUDA;
-  PlanKey key = {dev, mode, nr, nc, mode == MODE_GL ? G : 0, vec, tma ? 1 : 0, ctype, {}, ch};
+  PlanKey key = {dev, mode, nr, nc, mode == MODE_GL ? G : 0, vec, tma ? 1 : 0, ctype, {}, ch,
+                 false};
   if (mode == MODE_GL && ubounds) key.ubounds.assign(ubounds, ubounds + G + 1);
-  {
-    std::lock_guard<std::mutex> lk(g_plan_mu);
-    for (auto& e : g_plans)
-      if (e.first == key) { pl = e.second; return DROT_OK; }
-  }
+  if (g_plans.find(key, pl)) return DROT_OK;
   const int rc = make_plan_uncached(mode, nr, nc, G, vec, tma, ctype, pl,
                                     mode == MODE_GL ? ubounds : nullptr, ch);
-  if (rc == DROT_OK) {
-    std::lock_guard<std::mutex> lk(g_plan_mu);
-    if (g_plans.size() >= 64) g_plans.erase(g_plans.begin());
-    g_plans.emplace_back(key, pl);
-  }
+  if (rc == DROT_OK) g_plans.put(key, pl);
   return rc;
 }
 
@@ -426,6 +460,16 @@ static int choose_plan(int mode, int nr, int nc, int G, bool aligned4, Plan& pl,
   return make_plan(mode, nr, nc, G, aligned4 ? 4 : 1, false, pl, ctype, ubounds, ch);
 }
 
+// GL: the caller's row boundaries of the classes, or the reference's.
+static std::vector<int> row_bounds(int mode, int nr, int G, const int* ubounds) {
+  std::vector<int> bounds;
+  if (mode != MODE_GL) return bounds;
+  bounds.resize(G + 1);
+  if (ubounds) std::copy(ubounds, ubounds + G + 1, bounds.begin());
+  else group_bounds(nr, G, bounds.data());
+  return bounds;
+}
+
 // Resident plan of a problem whose tiles fit the chip (QR up to about 4100 x
 // 4100, beyond 1900 x 1900 in part; faster than the streaming kernel at every
 // size it takes, from 2.6x at 96 x 80 to 1.27x at 4000 x 4000), cached like the
@@ -437,37 +481,24 @@ static bool find_resident(int mode, int nr, int nc, int G, int ctype, const int*
   if (nr <= 0 || nc <= 0 || (mode == MODE_GL && (G <= 0 || G > kMaxGroups))) return false;
   if (!(find_choice(mode, nr, nc, G, ctype) == LaunchChoice())) return false;
   struct Entry {
-    PlanKey key;
-    bool check_all, fits;
+    bool fits;
     ResidentPlan plan;
   };
-  static std::mutex mu;
-  static std::vector<Entry> cache;
+  static PlanCache<Entry> cache;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return false;
-  PlanKey key = {dev, mode, nr, nc, mode == MODE_GL ? G : 0, 0, false, ctype, {}, LaunchChoice()};
+  PlanKey key = {dev, mode, nr, nc, mode == MODE_GL ? G : 0, 0, 0, ctype, {}, LaunchChoice(),
+                 check_all};
   if (mode == MODE_GL && ubounds) key.ubounds.assign(ubounds, ubounds + G + 1);
-  std::lock_guard<std::mutex> lk(mu);
-  for (auto& e : cache)
-    if (e.key == key && e.check_all == check_all) {
-      out = e.plan;
-      return e.fits;
-    }
   Entry e;
-  e.key = key;
-  e.check_all = check_all;
-  const DeviceInfo d = device_info();
-  if (!d.ok) return false;
-  std::vector<int> bounds;
-  if (mode == MODE_GL) {
-    bounds.resize(G + 1);
-    if (ubounds) std::copy(ubounds, ubounds + G + 1, bounds.begin());
-    else group_bounds(nr, G, bounds.data());
+  if (!cache.find(key, e)) {
+    const DeviceInfo d = device_info();
+    if (!d.ok) return false;
+    const std::vector<int> bounds = row_bounds(mode, nr, G, ubounds);
+    e.fits = resident_plan(mode, nr, nc, G, bounds.data(), ctype, check_all, d.sms, d.smem_optin,
+                           e.plan);
+    cache.put(key, e);
   }
-  e.fits = resident_plan(mode, nr, nc, G, bounds.data(), ctype, check_all, d.sms, d.smem_optin,
-                         e.plan);
-  if (cache.size() >= 64) cache.erase(cache.begin());
-  cache.push_back(e);
   out = e.plan;
   return e.fits;
 }
@@ -475,10 +506,6 @@ static bool find_resident(int mode, int nr, int nc, int G, int ctype, const int*
 static size_t scratch_bytes(int mode, int nr, int nc, int G, const int* ubounds = nullptr) {
   size_t best = 0;
   Plan pl;
-  ResidentPlan rp;
-  for (int ctype : {DROT_C_F32, DROT_C_BF16})
-    for (bool all : {false, true})
-      if (find_resident(mode, nr, nc, G, ctype, ubounds, all, rp)) best = std::max(best, rp.total);
   if (make_plan(mode, nr, nc, G, 4, true, pl, DROT_C_F32, ubounds) == DROT_OK)
     best = std::max(best, pl.total);
   if (make_plan(mode, nr, nc, G, 4, false, pl, DROT_C_F32, ubounds) == DROT_OK)
@@ -495,6 +522,11 @@ static size_t scratch_bytes(int mode, int nr, int nc, int G, const int* ubounds 
     if (ch.tma && ctype == DROT_C_F32 &&
         make_plan(mode, nr, nc, G, 4, true, pl, ctype, ubounds, ch) == DROT_OK)
       best = std::max(best, pl.total);
+  }
+  // and the resident kernel's words, whatever its tiles (the query searches none)
+  if (best > 0) {
+    const std::vector<int> bounds = row_bounds(mode, nr, G, ubounds);
+    best = std::max(best, resident_most_bytes(mode, nr, nc, G, bounds.data(), device_info().sms));
   }
   return best;
 }

@@ -54,6 +54,40 @@ static double tile_cost(bool gl, bool keep, int warps, int used, int cw, int gri
   return t;
 }
 
+// Workspace of a tiling: the statistics and flags, then the exchange words.
+static void resident_layout(ResidentPlan& pl) {
+  size_t off = 512;
+  auto take = [&](size_t words) {
+    const size_t at = off;
+    off = up256(off + words * sizeof(unsigned long long));
+    return at;
+  };
+  pl.off_massx = take(64);
+  pl.off_resx = take(4 * (size_t)kPairCopies * pl.grid);
+  pl.off_objx = take(2 * (size_t)pl.grid);
+  pl.off_rowx = take(2 * (size_t)pl.GR * pl.rt);
+  pl.off_colx = take(2 * (size_t)pl.GC * pl.ct);
+  pl.total = off;
+}
+
+size_t resident_most_bytes(int mode, int nr, int nc, int G, const int* bounds, int sms) {
+  // QR bands and chunks share the rows and columns out in whole vectors
+  ResidentPlan most;
+  most.grid = sms;
+  most.GR = most.GC = 1;
+  most.rt = nr + 4 * sms;
+  most.ct = nc + 4 * sms;
+  if (mode == MODE_GL) {
+    int h = 0;
+    for (int k = 0; k < G; ++k) h = std::max(h, bounds[k + 1] - (bounds[k] & ~3));
+    if (G > sms || h > 128 * kResidentMaxWarps) return 0;  // no tiling
+    most.GR = G;
+    most.rt = (h + 3) & ~3;
+  }
+  resident_layout(most);
+  return most.total;
+}
+
 bool resident_plan(int mode, int nr, int nc, int G, const int* bounds, int ctype, bool check_all,
                    int sms, int smem_optin, ResidentPlan& best) {
   const size_t csize = ctype == DROT_C_BF16 ? 2 : 4;
@@ -126,6 +160,7 @@ bool resident_plan(int mode, int nr, int nc, int G, const int* bounds, int ctype
     }
   }
   if (!found) return false;
+  resident_layout(best);
   const ResidentFn fn = resident_fn(mode, ctype, best.threads);
   int occ = 0;
   if (allow_shared_memory((const void*)fn) != cudaSuccess ||
@@ -135,18 +170,6 @@ bool resident_plan(int mode, int nr, int nc, int G, const int* bounds, int ctype
     cudaGetLastError();
     return false;
   }
-  size_t off = 512;
-  auto take = [&](size_t words) {
-    const size_t at = off;
-    off = up256(off + words * sizeof(unsigned long long));
-    return at;
-  };
-  best.off_massx = take(64);
-  best.off_resx = take(4 * (size_t)kPairCopies * best.grid);
-  best.off_objx = take(2 * (size_t)best.grid);
-  best.off_rowx = take(2 * (size_t)best.GR * best.rt);
-  best.off_colx = take(2 * (size_t)best.GC * best.ct);
-  best.total = off;
   return true;
 }
 

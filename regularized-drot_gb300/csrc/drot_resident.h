@@ -121,6 +121,9 @@ struct ResidentPlan {
 bool resident_plan(int mode, int nr, int nc, int G, const int* bounds, int ctype, bool check_all,
                    int sms, int smem_optin, ResidentPlan& pl);
 
+// At least the total of every plan of the problem.
+size_t resident_most_bytes(int mode, int nr, int nc, int G, const int* bounds, int sms);
+
 // Enqueues the solve; ws holds pl.total bytes, zeroed by the caller on the
 // same stream.  prm: problem fields set by the caller, plan fields by this.
 cudaError_t resident_launch(const ResidentPlan& pl, ResidentParams& prm,
