@@ -93,6 +93,7 @@ struct AdjParams {
   long long timeout_ns;
   int n_inst, n_seg, max_iters;
   int chunk;            // entries staged as digits at a time, a multiple of 32
+  int max_lines;        // lines of the largest instance
   double tol;
 };
 
@@ -142,15 +143,22 @@ __global__ void adj_mask_kernel(const AdjParams A) {
 // The matvec: for every line, the sum of the direction's entries over the set
 // bits of the line's mask words.  FP64 adds are slow on this part (a warp's add
 // takes 16 clocks of an SM), and adding set bit by set bit cost 110 us per CG
-// iteration at 11 M elements.  Here the sums are exact integer sums on the
-// tensor cores: the entries are written as 72-bit fixed-point numbers on the
-// scale of the instance's largest one (2^-72 of it is far below the rounding
-// of an FP64 sum), cut into 8 digits of 9 bits, and the product of the 0 / 1
-// mask (A: 16 lines x 16 entries) with the digits (B: 16 entries x 8 digits)
-// is an FP16 MMA with FP32 accumulation whose every partial sum is an integer
-// below 2^21 times 2^-24, so nothing is rounded.  The digit sums are added up
-// as 64-bit integers and rounded once, to FP64: at least the accuracy of the
-// FP64 sum, and independent of its order.
+// iteration at 11 M elements.  Here the sums are integer sums on the tensor
+// cores: the entries are written as 88-bit fixed-point numbers on the scale of
+// the instance's largest one, cut into 8 digits of 11 bits, and the product of
+// the 0 / 1 mask (A: 16 lines x 16 entries) with the digits (B: 16 entries x 8
+// digits) is an FP16 MMA with FP32 accumulation whose every partial sum is an
+// integer below 2^23 times 2^-24, so nothing is rounded.  The digit sums are
+// added up as 64-bit integers and rounded to FP64 (three times at most), and do
+// not depend on their order.
+//   Entries down to 2^-35 of the largest (its power of two, 2^E) are exact in
+// that, smaller ones cut below 2^(E-87).  The cut of a line's k entries, k
+// 2^(E-87) at most, is below one rounding of an FP64 sum of them unless they all
+// are small.  Those lines -- the line's own entry below 2^(E-34) and its sum
+// below k 2^(E-34): in a component of the support graph whose right-hand side is
+// small beside the others' -- are added entry by entry in FP64 instead
+// (line_walk), where an instance has entries that are cut at all: every line has
+// the accuracy of an FP64 sum of its own entries.
 //
 // One mask word (32 entries of a line) is two MMAs.  Their k indices are dealt
 // out so that a lane's operand is one AND: register r (0..3: the two halves of
@@ -175,16 +183,16 @@ __device__ __forceinline__ void mma_mask(float (&c)[4], unsigned a0, unsigned a1
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// |v| on the scale of exponent field emax as 72 bits in two halves of 36.
-__device__ __forceinline__ void to_fixed72(double v, int emax, unsigned long long& hi,
+// |v| on the scale of exponent field emax as 88 bits in two halves of 44.
+__device__ __forceinline__ void to_fixed88(double v, int emax, unsigned long long& hi,
                                            unsigned long long& lo) {
   const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
   const int e = (int)((bits >> 52) & 0x7ffu);
   const unsigned long long m = (bits & 0xfffffffffffffull) | 0x10000000000000ull;
   const int sh = emax - e;
-  const unsigned long long mask = (1ull << 36) - 1ull;
-  hi = sh < 37 ? m >> (17 + sh) : 0ull;
-  lo = (sh <= 19 ? m << (19 - sh) : (sh < 73 ? m >> (sh - 19) : 0ull)) & mask;
+  const unsigned long long mask = (1ull << 44) - 1ull;
+  hi = sh < 44 ? m >> (9 + sh) : 0ull;
+  lo = (sh <= 35 ? m << (35 - sh) : (sh < 88 ? m >> (sh - 35) : 0ull)) & mask;
   if (e == 0) hi = lo = 0ull;  // zero (and subnormal)
 }
 
@@ -197,8 +205,8 @@ __device__ __forceinline__ void stage_digits(const double* v, int n, int emax, u
     const int j0 = 32 * w + k, j1 = j0 + 16;
     const double v0 = j0 < n ? v[j0] : 0.0, v1 = j1 < n ? v[j1] : 0.0;
     unsigned long long h0, l0, h1, l1;
-    to_fixed72(v0, emax, h0, l0);
-    to_fixed72(v1, emax, h1, l1);
+    to_fixed88(v0, emax, h0, l0);
+    to_fixed88(v1, emax, h1, l1);
     // +- 2^-r, in both halves
     const unsigned r = k & 3, one = 0x3c00u - (r << 10);
     const unsigned sc = (one | (v0 < 0.0 ? 0x8000u : 0u)) |
@@ -207,12 +215,15 @@ __device__ __forceinline__ void stage_digits(const double* v, int n, int emax, u
     unsigned* const to = B + w * 128 + (k >> 2) * 4 + r;
 #pragma unroll
     for (int g = 0; g < 8; ++g) {
-      const int s = 27 - 9 * (g & 3);
-      const unsigned d0 = (unsigned)((g < 4 ? h0 : l0) >> s) & 0x1ffu;
-      const unsigned d1 = (unsigned)((g < 4 ? h1 : l1) >> s) & 0x1ffu;
-      // 1024 + digit has the digit as its low bits
-      const unsigned u = 0x64006400u | d0 | (d1 << 16);
-      const __half2 x = __hsub2(*reinterpret_cast<const __half2*>(&u), __half2half2(__ushort_as_half(0x6400)));
+      const int s = 33 - 11 * (g & 3);
+      const unsigned d0 = (unsigned)((g < 4 ? h0 : l0) >> s) & 0x7ffu;
+      const unsigned d1 = (unsigned)((g < 4 ? h1 : l1) >> s) & 0x7ffu;
+      // 1024 + the digit's low 10 bits has those as its low bits; less 1024 where
+      // the digit's top bit is clear
+      const unsigned u = 0x64006400u | (d0 & 0x3ffu) | (d1 & 0x3ffu) << 16;
+      const unsigned t = ((d0 >> 10) ^ 1u) * 0x6400u | ((d1 >> 10) ^ 1u) * 0x64000000u;
+      const __half2 x = __hsub2(*reinterpret_cast<const __half2*>(&u),
+                                *reinterpret_cast<const __half2*>(&t));
       const __half2 y = __hmul2(x, scale);
       to[g * 16] = *reinterpret_cast<const unsigned*>(&y);
     }
@@ -253,8 +264,8 @@ __device__ __forceinline__ void mask_sums(const unsigned* words, int stride, int
       }
     }
     // c[0], c[1]: digits 2 t, 2 t + 1 of line la; c[2], c[3]: of line lb
-    const long long sa = (long long)((int)(c[0] * 16777216.0f) * 512 + (int)(c[1] * 16777216.0f));
-    const long long sb = (long long)((int)(c[2] * 16777216.0f) * 512 + (int)(c[3] * 16777216.0f));
+    const long long sa = (long long)(int)(c[0] * 16777216.0f) * 2048 + (int)(c[1] * 16777216.0f);
+    const long long sb = (long long)(int)(c[2] * 16777216.0f) * 2048 + (int)(c[3] * 16777216.0f);
     if (la < n) atomicAdd(acc + 4 * la + t, (unsigned long long)sa);
     if (lb < n) atomicAdd(acc + 4 * lb + t, (unsigned long long)sb);
   }
@@ -262,10 +273,25 @@ __device__ __forceinline__ void mask_sums(const unsigned* words, int stride, int
 
 // The FP64 value of a line's digit sums.
 __device__ __forceinline__ double mask_sum_value(const unsigned long long* acc, int emax) {
-  double s = (double)(long long)acc[0] * 18014398509481984.0;        // 2^54
-  s = fma((double)(long long)acc[1], 68719476736.0, s);              // 2^36
-  s = fma((double)(long long)acc[2], 262144.0, s) + (double)(long long)acc[3];
-  return emax == 0x7ff ? __longlong_as_double(0x7ff8000000000000ll) : scalbn(s, emax - 1094);
+  double s = (double)(long long)acc[0] * 73786976294838206464.0;     // 2^66
+  s = fma((double)(long long)acc[1], 17592186044416.0, s);           // 2^44
+  s = fma((double)(long long)acc[2], 4194304.0, s) + (double)(long long)acc[3];
+  return emax == 0x7ff ? __longlong_as_double(0x7ff8000000000000ll) : scalbn(s, emax - 1110);
+}
+
+// A warp: the sum over the set bits of a line's nw mask words of the entries src,
+// in FP64.  nz: a bit per entry, set where it is not zero; src's first is bit
+// `shift` of nz[0].
+__device__ __noinline__ double line_walk(const unsigned* words, int nw, const double* src,
+                                         const unsigned* nz, int shift) {
+  double s = 0.0;
+  bool any = false;
+  for (int w = threadIdx.x & 31; w < nw; w += 32) {
+    unsigned m = __ldg(words + w) & __funnelshift_r(nz[w], nz[w + 1], shift);
+    any |= m != 0u;
+    for (; m; m &= m - 1u) s += src[32 * w + __ffs(m) - 1];
+  }
+  return __any_sync(0xffffffffu, any) ? warp_sum_d(s) : 0.0;
 }
 
 // Degree of line l and the right-hand side entry of the adjoint system: the
@@ -348,7 +374,9 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adj_pcg_kernel(const AdjParams
   unsigned* const digits = reinterpret_cast<unsigned*>(acc + 4 * kAdjBlock);  // [A.chunk] entries
   double* const sv = reinterpret_cast<double*>(
       adj_smem + 32 * kAdjBlock + (size_t)kAdjDigitBytes * A.chunk);  // the staged direction
+  unsigned* const nz = reinterpret_cast<unsigned*>(sv + A.max_lines);  // bits of its nonzeros
   __shared__ int s_flag, s_emax;
+  __shared__ unsigned s_emin;
   __shared__ double s_red[32 + 1];
   __shared__ double s_part[2][16];
   __shared__ double s_step;  // beta, then alpha
@@ -414,6 +442,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adj_pcg_kernel(const AdjParams
         if (lane == 0) s_step = ry / ryp;
       } else if (threadIdx.x == 64) {
         s_emax = 0;
+        s_emin = 0xfffu;
       }
       __syncthreads();
       if (s_done) {
@@ -427,7 +456,10 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adj_pcg_kernel(const AdjParams
       const int nv = I.nr + I.nc;
       // Stage d = y + beta d_old for the whole instance: a thread takes 4
       // entries and issues their loads before using any.
-      unsigned top = 0u;  // the largest magnitude's upper word
+      // upper words of the largest magnitude and of the smallest that is not zero
+      // (less one, which puts zero last; an upper word of zero beside a lower one
+      // that is not is a subnormal, which counts as zero)
+      unsigned top = 0u, bottom = 0xffffffffu;
       for (int t0 = threadIdx.x; t0 < nv; t0 += 4 * blockDim.x) {
         double yv[4], dv0[4];
 #pragma unroll
@@ -443,14 +475,30 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adj_pcg_kernel(const AdjParams
           if (t >= nv) break;
           const double dv = it == 0 ? yv[u] : fma(beta, dv0[u], yv[u]);
           sv[t] = dv;
-          top = max(top, (unsigned)__double2hiint(dv) & 0x7fffffffu);
+          const unsigned size = (unsigned)__double2hiint(dv) & 0x7fffffffu;
+          top = max(top, size);
+          bottom = min(bottom, size - 1u);
           if (t >= S.l0 && t < S.l1) dcur[I.v_off + t] = dv;
         }
       }
       top = __reduce_max_sync(0xffffffffu, top);
-      if (lane == 0) atomicMax(&s_emax, (int)(top >> 20));
+      bottom = __reduce_min_sync(0xffffffffu, bottom);
+      if (lane == 0) {
+        atomicMax(&s_emax, (int)(top >> 20));
+        atomicMin(&s_emin, bottom >> 20);
+      }
       __syncthreads();
       const int emax = s_emax;
+      // 2^(E-34) of the lines that are added in FP64, where entries are cut
+      const double low = emax > 36 && emax < 0x7ff && s_emin < (unsigned)(emax - 35)
+                             ? __hiloint2double((emax - 34) << 20, 0) : 0.0;
+      if (low > 0.0) {  // the nonzeros of the direction, for line_walk
+        for (int t0 = 32 * warp; t0 < nv; t0 += blockDim.x) {
+          const unsigned b = __ballot_sync(0xffffffffu, t0 + lane < nv && sv[t0 + lane] != 0.0);
+          if (lane == 0) nz[t0 >> 5] = b;
+        }
+        __syncthreads();
+      }
       double dq = 0.0;
       // the segment's rows against the column entries, then its columns
       // against the row entries
@@ -472,12 +520,28 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adj_pcg_kernel(const AdjParams
                       digits, acc);
             __syncthreads();
           }
-          for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            const int l = b0 + i, gi = I.v_off + l;
-            const double dl = sv[l];
-            const double qv = fma(__ldcg(A.deg + gi), dl, mask_sum_value(acc + 4 * i, emax));
-            A.q[gi] = qv;
-            dq += dl * qv;
+          const unsigned* const bits = side ? nz : nz + (I.nr >> 5);
+          const int shift = side ? 0 : I.nr & 31;
+          for (int i0 = 32 * warp; i0 < n; i0 += blockDim.x) {
+            const int i = i0 + lane, l = b0 + i, gi = I.v_off + l;
+            double dl = 0.0, dg = 0.0, sum = 0.0;
+            if (i < n) {
+              dl = sv[l];
+              dg = __ldcg(A.deg + gi);
+              sum = mask_sum_value(acc + 4 * i, emax);
+            }
+            unsigned todo = __ballot_sync(0xffffffffu, fabs(dl) < low && fabs(sum) < dg * low);
+            for (; todo; todo &= todo - 1u) {
+              const int k = __ffs(todo) - 1;
+              const double t = line_walk(words + (long long)(b0 + i0 + k) * stride, (K + 31) >> 5,
+                                         src, bits, shift);
+              if (lane == k) sum = t;
+            }
+            if (i < n) {
+              const double qv = fma(dg, dl, sum);
+              A.q[gi] = qv;
+              dq += dl * qv;
+            }
           }
           __syncthreads();
         }
@@ -622,7 +686,7 @@ using namespace drot;
 namespace {
 
 struct AdjLayout {
-  int grid = 0, threads = kAdjThreads, n_seg = 0, V = 0, chunk = 0;
+  int grid = 0, threads = kAdjThreads, n_seg = 0, V = 0, chunk = 0, max_lines = 0;
   size_t smem = 0;
   std::vector<AdjInst> inst;
   std::vector<AdjSeg> seg;
@@ -683,7 +747,9 @@ int adj_layout(int n_inst, const drot_adjoint_instance* d, AdjLayout& L) {
     return DROT_ERR_CUDA;
   // The direction, the line sums, and as many of the digits as fit beside them
   // (all of one side for up to 4096 rows or columns).
-  L.smem = sizeof(double) * (size_t)maxv + 32 * (size_t)kAdjBlock;
+  L.max_lines = maxv;
+  L.smem = sizeof(double) * (size_t)maxv + sizeof(unsigned) * ((size_t)maxv / 32 + 2) +
+           32 * (size_t)kAdjBlock;
   const long long room = ((long long)optin - 2048 - (long long)L.smem) / kAdjDigitBytes;
   L.chunk = (int)std::min<long long>(std::min(kAdjChunk, (maxk + 31) & ~31), room & ~31LL);
   if (L.chunk < 32) return DROT_ERR_UNSUPPORTED;
@@ -795,6 +861,7 @@ static void adj_params(const AdjLayout& L, char* ws, AdjParams& A) {
   A.deg = vec + 5 * (size_t)L.V;
   A.y = vec + 6 * (size_t)L.V;
   A.chunk = L.chunk;
+  A.max_lines = L.max_lines;
   A.mcol = (unsigned*)(ws + L.off_mcol);
   A.mrow = (unsigned*)(ws + L.off_mrow);
   A.inst = (const AdjInst*)(ws + L.off_inst);
