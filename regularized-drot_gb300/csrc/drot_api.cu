@@ -115,6 +115,7 @@ static inline size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAl
 struct Plan {
   int mode = 0, vec = 4, kv = 4, wt = 1, threads = 256, nbands = 1, P = 1, grid = 1, nsb = 1;
   int band_h = 0, ns = 1, p2_smem = 0, p2_cap_r = 0, p2_cap_c = 0, ctype = DROT_C_F32;
+  int levels = 0;
   bool tma = false;
   size_t smem = 0;
   std::vector<int> bounds;
@@ -277,7 +278,17 @@ static int make_plan_uncached(int mode, int nr, int nc, int G, int vec, bool tma
       pl.ns = 1;
     }
     pl.threads = 32 * warps;
-    pl.smem = solve_smem_bytes(warps, pl.wt, S, pl.ns, tma);
+    // GL beyond L2: four blocks of columns.  Two where the sums that wait would
+    // take shared memory from the L1 cache that holds the spills of the 8-vector
+    // kernel with a float cost: 10000 x 10000 in 2 classes 221 us per iteration
+    // with four blocks, 215 with two (7000 x 6000 in 7 with a BF16 cost 71, 74.5;
+    // eight blocks of 4-vector teams, 6000 x 5000 in 3: 65.9 against 65.2).
+    const double x_and_c = (double)nr * (double)nc * (ctype == DROT_C_BF16 ? 6.0 : 8.0);
+    pl.levels = 0;
+    if (mode == MODE_GL && !tma && x_and_c > (double)dev.l2)
+      pl.levels = pl.kv == 8 && ctype == DROT_C_F32 ? 1 : 2;
+    if (solve_smem_bytes(warps, pl.wt, S, pl.ns, tma, 0, pl.levels) > budget) pl.levels = 0;
+    pl.smem = solve_smem_bytes(warps, pl.wt, S, pl.ns, tma, 0, pl.levels);
     if (pl.smem > budget) return DROT_ERR_UNSUPPORTED;
     if (pl.smem > 48 * 1024 && allow_shared_memory((const void*)fn) != cudaSuccess)
       return DROT_ERR_CUDA;
@@ -315,7 +326,7 @@ static int make_plan_uncached(int mode, int nr, int nc, int G, int vec, bool tma
   const int capc = ((nc + pl.grid - 1) / pl.grid + 3) & ~3;
   const int p2f = 3 * (capr + capc);
   const int warps = pl.threads / 32;
-  const size_t smem2 = solve_smem_bytes(warps, pl.wt, S, pl.ns, tma, p2f);
+  const size_t smem2 = solve_smem_bytes(warps, pl.wt, S, pl.ns, tma, p2f, pl.levels);
   pl.p2_smem = 0;
   pl.p2_cap_r = pl.p2_cap_c = 0;
   if ((size_t)p2f * sizeof(float) <= 48 * 1024 && smem2 <= budget) {
@@ -587,7 +598,7 @@ struct SolveArgs {
   cudaStream_t stream;
   const int* bounds = nullptr;  // GL: caller's group boundaries (null: the reference's)
   int stop_every = 0, stop_le = 0;  // numpy-API stop rule (QR)
-  int first = 0;  // iterations before this call, where that is known
+  int first = 0;  // iterations before this call, where that is known (no result depends on it)
 };
 
 static int read_stats(const void* ws, drot_result* r, cudaStream_t stream) {
@@ -735,6 +746,7 @@ static int run_solve(const SolveArgs& A, drot_result* result) {
   prm.nr_rcp = (float)(1.0 / (double)(float)A.nr);
   prm.max_iters = A.max_iters;
   prm.first = A.first;
+  prm.levels = pl.levels;
   prm.stop_every = A.stop_every;
   prm.stop_le = A.stop_le;
   prm.res2_stop = res2_threshold(A.eps, A.mode == MODE_QR && !A.stop_le);

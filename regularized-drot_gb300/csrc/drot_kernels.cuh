@@ -93,7 +93,8 @@ struct SolveParams {
                        // its square root of the absolute tolerance eps
                        // (set by the host)
   int max_iters;
-  int first;           // iterations before this launch (parity: the order of the columns)
+  int first;           // iterations before this launch (which way it walks the columns)
+  int levels;          // GL: 1 << levels blocks of columns, walked either way (0: forwards)
   int stop_every;      // QR: test every iteration (numpy-API loop), not only even ones
   int stop_le;         // QR: stop on residual <= eps (numpy-API loop) instead of < eps
   int nbands;          // QR: row bands; GL: groups
@@ -597,6 +598,8 @@ __device__ __forceinline__ void reduce_partials(int r0, int r1, int k0, int k1,
 // Dynamic shared memory of the solve kernel (must match the device layout).
 //   ring    TMA: W * ns * 2 * S floats (stage: X segment, C segment)
 //           reg: W * S floats (row-partial staging only)
+//   stash   GL, per level: W * S row partials (the first level's are the ring's),
+//           W * 32 mass and objective pairs
 //   f1s     Wt * S floats (phi1 of the band rows)
 //   st2     3 * (cap_r + cap_c) floats when the phase-2 state is in shared
 //           memory (p, a, staged phi1 of the CTA's rows; q, b, phi2 of its columns)
@@ -604,8 +607,10 @@ __device__ __forceinline__ void reduce_partials(int r0, int r1, int k0, int k1,
 //   nslot   2 * W float pairs (per-warp objective sums; GL team norms)
 //   mbar    W * ns uint64 (TMA only)
 __host__ __device__ constexpr size_t solve_smem_bytes(int warps, int wt, int S, int ns, bool tma,
-                                                      int p2_floats = 0) {
+                                                      int p2_floats = 0, int levels = 0) {
   return sizeof(float) * (size_t)warps * S * (tma ? 2 * ns : 1) + sizeof(float) * (size_t)wt * S +
+         (levels ? (levels - 1) * sizeof(float) * (size_t)warps * S : 0) +
+         32 * sizeof(float4) * (size_t)levels * warps +
          sizeof(float) * (size_t)p2_floats + sizeof(double) * (warps + 1) +
          sizeof(double) * 2 * warps + (tma ? sizeof(uint64_t) * (size_t)warps * ns : 0);
 }
@@ -630,7 +635,11 @@ drot_solve_kernel(const SolveParams P) {
   const int capc = P.p2_smem ? P.p2_cap_c : 0;
   float* ring = reinterpret_cast<float*>(smem_raw);
   float* red = ring;  // row-partial staging aliases the ring (ring idle then)
-  float* f1s = ring + (size_t)W * S * (TMA ? 2 * NS : 1);
+  constexpr bool BLOCKS = MODE == MODE_GL && !TMA;
+  const int levels = BLOCKS ? P.levels : 0;
+  float4* stash2 = reinterpret_cast<float4*>(
+      ring + (size_t)W * S * (TMA ? 2 * NS : max(levels, 1)));
+  float* f1s = reinterpret_cast<float*>(stash2 + (size_t)levels * W * 32);
   float* s_p = f1s + (size_t)Wt * S;
   float* s_a = s_p + capr;
   float* s_t1 = s_a + capr;
@@ -780,15 +789,19 @@ drot_solve_kernel(const SolveParams P) {
     // exact float pairs (TwoSum); FP64 only once per iteration.
     float ms_hi = 0.0f, ms_lo = 0.0f, ob_hi = 0.0f, ob_lo = 0.0f;
     bool wfail = false;
-    // Odd iterations walk the warp's columns backwards: the columns that the
-    // last iteration touched last are still in L2 when X + C exceed it.  us
-    // per iteration, forwards only -> alternating: QR 10000 x 10000 168 -> 162,
-    // GL 6000 x 5000 69 -> 63, 3000 x 3000 (fits L2) the same.  (Eviction
+    // Every other iteration walks the warp's columns the other way: the columns
+    // that the last iteration touched last are still in L2 when X + C exceed it.
+    // us per iteration, forwards only -> alternating: QR 10000 x 10000 168 -> 162,
+    // GL 6000 x 5000 70 -> 65, 3000 x 3000 (fits L2) the same.  (Eviction
     // priorities instead -- evict_last on the first columns of every CTA,
-    // evict_first on the rest -- measured 170 and 62.5.)  The order is that of
-    // the whole solve's iteration count where the caller knows it, so
-    // recomputing single iterations gives the same sums.
-    const bool back = MODE == MODE_QR ? !even : ((it + P.first) & 1) != 0;
+    // evict_first on the rest -- measured 170 and 62.5.)
+    //   A QR solve is split into launches at even counts only, so it takes the
+    // columns singly, backwards on odd iterations.  GL may be split anywhere, and
+    // one launch has to give the bits of several: its sums do not depend on the
+    // way.  The columns form 1 << levels blocks, each summed forwards, and the
+    // blocks' sums are added as a binary tree; walked backwards the operands of
+    // every addition change places, no more.
+    const bool back = MODE == MODE_QR ? !even : BLOCKS && ((it + P.first) & 1) != 0;
 
     // One column of the band per team step.  EV selects the QR step that
     // reads C and stores the folded value X^ - sC (kernel_qr.hpp:171-278);
@@ -801,7 +814,9 @@ drot_solve_kernel(const SolveParams P) {
       const int ncw = (c1 - c0 - team + nteams - 1) / nteams;  // columns of this warp
       const uint32_t tx_bytes = seg_bytes * (WITH_C ? 2u : 1u);
       // Column n of the warp in this iteration's order.
-      auto col_of = [&](int n) { return c0 + team + (back ? ncw - 1 - n : n) * nteams; };
+      auto col_of = [&](int n) {
+        return c0 + team + (MODE == MODE_QR && back ? ncw - 1 - n : n) * nteams;
+      };
       uint32_t issued = pipe_cnt;
       auto issue = [&](int n) {  // lane 0: fetch column n of this warp into its stage
         const int jn = col_of(n);
@@ -1118,12 +1133,50 @@ drot_solve_kernel(const SolveParams P) {
           finish(ja, xa, cz, 0);
           if (two) finish(jb, xb, cz, 0);
         }
-      } else {
+      } else if constexpr (!BLOCKS) {
         int par = 0;
         for (int n = 0; n < ncw; ++n, par ^= 1) {
           float xv[KV][VEC], cv[KV][VEC];
           load_reg(col_of(n), xv, cv);
           finish(col_of(n), xv, cv, par);
+        }
+      } else {
+        const int blocks = 1 << levels;
+        int par = 0;
+        for (int i = 0; i < blocks; ++i) {
+          const int b = back ? blocks - 1 - i : i;
+          const int n1 = ncw * (b + 1) / blocks;
+          for (int n = ncw * b / blocks; n < n1; ++n, par ^= 1) {
+            float xv[KV][VEC], cv[KV][VEC];
+            load_reg(col_of(n), xv, cv);
+            finish(col_of(n), xv, cv, par);
+          }
+          // The block's sums meet those of the subtrees that wait (a binary
+          // counter), then wait themselves.
+          int l = 0;
+          for (; (i >> l) & 1; ++l) {
+            const float* const to = ring + ((size_t)l * W + warp) * S + lane * VEC;
+#pragma unroll
+            for (int v = 0; v < KV; ++v)
+#pragma unroll
+              for (int e = 0; e < VEC; ++e) acc[v][e] += to[v * SV + e];
+            const float4 w = stash2[((size_t)l * W + warp) * 32 + lane];
+            const fpair m = fp_add(fpair{ms_hi, ms_lo}, fpair{w.x, w.y});
+            const fpair o = fp_add(fpair{ob_hi, ob_lo}, fpair{w.z, w.w});
+            ms_hi = m.hi; ms_lo = m.lo;
+            ob_hi = o.hi; ob_lo = o.lo;
+          }
+          if (i + 1 < blocks) {
+            float* const to = ring + ((size_t)l * W + warp) * S + lane * VEC;
+#pragma unroll
+            for (int v = 0; v < KV; ++v) {
+              store_vec<VEC>(to + v * SV, acc[v]);
+#pragma unroll
+              for (int e = 0; e < VEC; ++e) acc[v][e] = 0.0f;
+            }
+            stash2[((size_t)l * W + warp) * 32 + lane] = make_float4(ms_hi, ms_lo, ob_hi, ob_lo);
+            ms_hi = ms_lo = ob_hi = ob_lo = 0.0f;
+          }
         }
       }
     };
