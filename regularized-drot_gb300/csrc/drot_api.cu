@@ -648,7 +648,7 @@ static int run_resident(const SolveArgs& A, const ResidentPlan& pl, const void* 
   char* const ws = (char*)A.ws;
   prm.stats = (DeviceStats*)ws;
   prm.abort_flag = (int*)(ws + 256 + 64);
-  prm.odd_flag = (int*)(ws + 256 + 128);
+  prm.over_flag = (int*)(ws + 256 + 128);
   prm.timer_cta = getenv("DROT_TIMER_CTA") ? atoi(getenv("DROT_TIMER_CTA")) : 0;
   if (prm.timer_cta < 0 || prm.timer_cta >= pl.grid) prm.timer_cta = 0;
   prm.timeout_ns = barrier_timeout_ns();

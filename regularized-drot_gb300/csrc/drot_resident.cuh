@@ -47,9 +47,10 @@
 //   Fixed point: a total has an error of at most GC 2^-47, below the rounding
 // of the FP32 duals it updates.  A CTA whose mass would exceed the words'
 // range (or is not finite) adds a poison count to the mass word instead; then
-// every CTA repeats the round with 8 fraction bits fewer (or with counts of
-// infinities and NaNs), so the arithmetic depends on the data of the
-// iteration alone and a solve split into segments gives the same bits.
+// every CTA repeats the round with 8 fraction bits fewer (or, where all finite
+// sums fit, adds a round of counts of infinities and NaNs), so the arithmetic
+// depends on the data of the iteration alone and a solve split into segments gives
+// the same bits.
 //   The squared residual is published as tagged words {value, tag}, in two
 // slots that take turns (drot_exchange.h: residual_slot, with the order that
 // makes that safe), and read during the next iteration, whose X-update runs
@@ -224,7 +225,8 @@ struct LLWait {
 
 // Fixed-point words: 46 fraction bits for rows and columns, 38 for the mass,
 // 8 fewer per level.  In a class round (level < 0) a contribution counts a
-// NaN (bits 40 up) or an infinity (bits 20 up).
+// NaN (bits 40 up) or an infinity (bits 20 up); it follows a round that held the
+// finite sums, and replaces the others.
 constexpr int kRowBits = 46, kMassBits = 38, kLevelBits = 8;
 constexpr unsigned long long kCountOne = 1ull << 56, kPoisonOne = 1ull << 48;
 
@@ -880,7 +882,7 @@ __device__ __forceinline__ void resident_solve(const ResidentParams& P, const in
             if (level < 0) {
               n += class_word(v);
             } else {
-              const bool fin = v < 3.402823466e38f;
+              const bool fin = v <= 3.402823466e38f;
               odd_value |= !fin;
               const float f = fin ? v * upm : 0.0f;
               over |= !(f < (float)most);
@@ -900,8 +902,8 @@ __device__ __forceinline__ void resident_solve(const ResidentParams& P, const in
           }
           unsigned long long* const mw = P.massx + 32 * rp;
           if (lane == 0) {
-            if (odd_value) {
-              atomicExch(P.odd_flag, it + 1);
+            if (over) {
+              atomicExch(P.over_flag, (int)(rd + 1u));
               __threadfence();
             }
             if (!mute)
@@ -918,7 +920,7 @@ __device__ __forceinline__ void resident_solve(const ResidentParams& P, const in
               sg = class_value(d & (kPoisonOne - 1ull));
             } else if ((d >> 48) & 0xffull) {
               __threadfence();
-              next = ld_volatile_i32(P.odd_flag) == it + 1 ? -1 : level + 1;
+              next = ld_volatile_i32(P.over_flag) == (int)(rd + 1u) ? level + 1 : -1;
             } else {
               sg = from_fixed(d & (kPoisonOne - 1ull)) * pow2f(kLevelBits * level - kMassBits);
             }
@@ -995,6 +997,11 @@ __device__ __forceinline__ void resident_solve(const ResidentParams& P, const in
               tot[u] = level < 0 ? class_value(n)
                                  : from_fixed(n) * pow2f(kLevelBits * level - kRowBits);
             }
+            if (level < 0) {
+              if (np == 1 || tot[u] == 0.0f) continue;  // finite: the round before updated it
+              if constexpr (LEAN) dual[u] = s_prev[i];
+              else dual[u] = dual_prev[u];
+            }
             const float rs = tot[u] - (LEAN ? s_marg[i] : marg[u]);
             if constexpr (LEAN) s_prev[i] = dual[u];
             else dual_prev[u] = dual[u];
@@ -1023,13 +1030,16 @@ __device__ __forceinline__ void resident_solve(const ResidentParams& P, const in
         if (decided && s_stop) stop_it = pend;
         break;
       }
-      // The words could not hold this round: again on a coarser scale.
+      // The words could not hold this round: again on a coarser scale, or the
+      // sums that are not finite.
       level = next;
+      if (next > 0) {
 #pragma unroll
-      for (int u = 0; u < NI; ++u) {
-        const int i = tid + u * IT;
-        if constexpr (!LEAN) dual[u] = dual_prev[u];
-        else if (warp < res_warp && i < n_items) dual[u] = s_prev[i];
+        for (int u = 0; u < NI; ++u) {
+          const int i = tid + u * IT;
+          if constexpr (!LEAN) dual[u] = dual_prev[u];
+          else if (warp < res_warp && i < n_items) dual[u] = s_prev[i];
+        }
       }
       __syncthreads();
     }
@@ -1375,7 +1385,7 @@ drot_resident_batch_kernel(const __grid_constant__ ResidentBatch B) {
       prm.rowx = B.words + I.rowx_off;
       prm.colx = B.words + I.colx_off;
       prm.abort_flag = B.abort_flag;
-      prm.odd_flag = reinterpret_cast<int*>(prm.massx + 64);
+      prm.over_flag = reinterpret_cast<int*>(prm.massx + 64);
       prm.record = B.records + I.index;
       prm.beat = reinterpret_cast<unsigned*>(B.sched + kSchedBeat);
       prm.stall_cta = B.stall_cta == me ? tile : -1;  // the test hook names a CTA of the launch

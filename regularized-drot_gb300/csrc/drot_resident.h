@@ -37,7 +37,7 @@ struct ResidentParams {
   unsigned long long* massx;        // [2] of them, 256 bytes apart
   unsigned long long* resx;         // [2 slots][kPairCopies][grid][2] tagged (hi, lo)
   unsigned long long* objx;         // [grid][2]
-  int *abort_flag, *odd_flag;       // odd_flag: iteration + 1 of a sum that was not finite
+  int *abort_flag, *over_flag;      // over_flag: round + 1 of a mass beyond the words' range
   DeviceStats* stats;
   struct BatchRecord* record;  // batches: instead of stats
   int alpha_stride;            // batches: floats between the parity slots of alpha
