@@ -33,6 +33,16 @@ namespace drot {
 
 typedef void (*SolveFn)(const SolveParams);
 
+template <typename CT>
+static SolveFn kernel_blocks(int vec, int kv) {
+  if (vec != 4) return nullptr;
+  if (kv == 1) return drot_solve_kernel<MODE_GL, 4, 1, false, CT, true>;
+  if (kv == 2) return drot_solve_kernel<MODE_GL, 4, 2, false, CT, true>;
+  if (kv == 4) return drot_solve_kernel<MODE_GL, 4, 4, false, CT, true>;
+  if (kv == 8) return drot_solve_kernel<MODE_GL, 4, 8, false, CT, true>;
+  return nullptr;
+}
+
 template <int MODE, bool TMA, typename CT>
 static SolveFn kernel_kv(int vec, int kv) {
   if constexpr (TMA) {
@@ -64,8 +74,11 @@ static SolveFn kernel_kv(int vec, int kv) {
 }
 
 // Kernel instance for (mode, vector width, vectors per lane, data path, cost
-// type).  The TMA ring exists for float costs only.
-static SolveFn kernel_for(int mode, int vec, int kv, bool tma, int ctype = DROT_C_F32) {
+// type, GL columns in blocks).  The TMA ring exists for float costs only.
+static SolveFn kernel_for(int mode, int vec, int kv, bool tma, int ctype, bool blocks) {
+  if (blocks)
+    return ctype == DROT_C_BF16 ? kernel_blocks<__nv_bfloat16>(vec, kv)
+                                : kernel_blocks<float>(vec, kv);
   if (ctype == DROT_C_BF16) {
     if (tma) return nullptr;
     return mode == MODE_QR ? kernel_kv<MODE_QR, false, __nv_bfloat16>(vec, kv)
@@ -174,6 +187,11 @@ struct LaunchChoice {
   }
 };
 
+// Share of L2 that X + C may take before the GL kernel walks its columns both ways
+// (forwards, both ways in us per iteration: 3400 x 3000 in 5 classes, 82 MB, 27.6,
+// 28.9; 3500 x 3300 in 2, 92 MB, 30.9, 30.3; 4000 x 3500 in 2, 112 MB, 36.8, 33.5).
+constexpr double kBlocksFromL2 = 0.75;
+
 // Build the launch plan for one data path (tma: shared-memory TMA ring, else
 // register loads).  Returns a drot_status.
 static int make_plan_uncached(int mode, int nr, int nc, int G, int vec, bool tma, int ctype,
@@ -245,7 +263,15 @@ static int make_plan_uncached(int mode, int nr, int nc, int G, int vec, bool tma
     }
   }
   const int S = SV * pl.kv;
-  SolveFn fn = kernel_for(mode, vec, pl.kv, tma, ctype);
+  // GL beyond L2, or nearly: four blocks of columns.  Two where the sums that wait
+  // would take shared memory from the L1 cache that holds the spills of the
+  // 8-vector kernel with a float cost: 10000 x 10000 in 2 classes 221 us per
+  // iteration with four blocks, 215 with two (7000 x 6000 in 7 with a BF16 cost 71,
+  // 74.5; eight blocks of 4-vector teams, 6000 x 5000 in 3: 65.9 against 65.2).
+  const double x_and_c = (double)nr * (double)nc * (ctype == DROT_C_BF16 ? 6.0 : 8.0);
+  if (mode == MODE_GL && !tma && vec == 4 && x_and_c > kBlocksFromL2 * (double)dev.l2)
+    pl.levels = pl.kv == 8 && ctype == DROT_C_F32 ? 1 : 2;
+  SolveFn fn = kernel_for(mode, vec, pl.kv, tma, ctype, pl.levels > 0);
   if (!fn) return DROT_ERR_UNSUPPORTED;
   pl.ctype = ctype;
   // TMA ring: 1 (default) or 2 CTAs per SM share the shared memory.
@@ -278,16 +304,11 @@ static int make_plan_uncached(int mode, int nr, int nc, int G, int vec, bool tma
       pl.ns = 1;
     }
     pl.threads = 32 * warps;
-    // GL beyond L2: four blocks of columns.  Two where the sums that wait would
-    // take shared memory from the L1 cache that holds the spills of the 8-vector
-    // kernel with a float cost: 10000 x 10000 in 2 classes 221 us per iteration
-    // with four blocks, 215 with two (7000 x 6000 in 7 with a BF16 cost 71, 74.5;
-    // eight blocks of 4-vector teams, 6000 x 5000 in 3: 65.9 against 65.2).
-    const double x_and_c = (double)nr * (double)nc * (ctype == DROT_C_BF16 ? 6.0 : 8.0);
-    pl.levels = 0;
-    if (mode == MODE_GL && !tma && x_and_c > (double)dev.l2)
-      pl.levels = pl.kv == 8 && ctype == DROT_C_F32 ? 1 : 2;
-    if (solve_smem_bytes(warps, pl.wt, S, pl.ns, tma, 0, pl.levels) > budget) pl.levels = 0;
+    if (pl.levels > 0 &&
+        solve_smem_bytes(warps, pl.wt, S, pl.ns, tma, 0, pl.levels) > budget) {
+      pl.levels = 0;
+      fn = kernel_for(mode, vec, pl.kv, tma, ctype, false);
+    }
     pl.smem = solve_smem_bytes(warps, pl.wt, S, pl.ns, tma, 0, pl.levels);
     if (pl.smem > budget) return DROT_ERR_UNSUPPORTED;
     if (pl.smem > 48 * 1024 && allow_shared_memory((const void*)fn) != cudaSuccess)
@@ -774,7 +795,7 @@ static int run_solve(const SolveArgs& A, drot_result* result) {
 
   if (cudaMemsetAsync(ws, 0, 512, A.stream) != cudaSuccess) return DROT_ERR_CUDA;
   if (repack && copy_in(A, cpad, xpad, ldp) != DROT_OK) return DROT_ERR_CUDA;
-  SolveFn fn = kernel_for(A.mode, pl.vec, pl.kv, pl.tma, pl.ctype);
+  SolveFn fn = kernel_for(A.mode, pl.vec, pl.kv, pl.tma, pl.ctype, pl.levels > 0);
   if (pl.smem > 48 * 1024 && allow_shared_memory((const void*)fn) != cudaSuccess)
     return DROT_ERR_CUDA;
   void* args[] = {(void*)&prm};

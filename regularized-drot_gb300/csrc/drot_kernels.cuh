@@ -619,9 +619,12 @@ __host__ __device__ constexpr size_t solve_smem_bytes(int warps, int wt, int S, 
 // The solve kernel
 // ---------------------------------------------------------------------------
 
-template <int MODE, int VEC, int KV, bool TMA, typename CT = float>
+// BLOCKS: GL, the columns in blocks that are walked either way (a kernel of its
+// own: with both loops in one, problems within L2 were 3 % slower).
+template <int MODE, int VEC, int KV, bool TMA, typename CT = float, bool BLOCKS = false>
 __global__ void __launch_bounds__(512, 1)
 drot_solve_kernel(const SolveParams P) {
+  static_assert(!BLOCKS || (MODE == MODE_GL && !TMA), "blocks are the GL register path's");
   static_assert(!TMA || VEC == 4, "the TMA path moves 16-byte vectors");
   static_assert(!TMA || std::is_same<CT, float>::value, "the TMA path streams float costs");
   const CT* const cbase = reinterpret_cast<const CT*>(P.c);
@@ -635,7 +638,6 @@ drot_solve_kernel(const SolveParams P) {
   const int capc = P.p2_smem ? P.p2_cap_c : 0;
   float* ring = reinterpret_cast<float*>(smem_raw);
   float* red = ring;  // row-partial staging aliases the ring (ring idle then)
-  constexpr bool BLOCKS = MODE == MODE_GL && !TMA;
   const int levels = BLOCKS ? P.levels : 0;
   float4* stash2 = reinterpret_cast<float4*>(
       ring + (size_t)W * S * (TMA ? 2 * NS : max(levels, 1)));
