@@ -24,13 +24,16 @@ forward + backward of the differentiable OT loss over one batch:
   plain        the same 64 instances one at a time with the drop-in
                operator's entry point (reg_drot.solve_qr: FP32, forward
                only); batched_over_plain = value / plain.
-  roofline     drot_resident_batch_kernel, the dominant kernel of the step:
-               algorithmic bytes of its launch (12 B per element on the
+  roofline     drot_resident_batch_kernel, the dominant kernel of the step: the
+               HBM bytes it moves (the bytes of streaming every active
+               instance once per iteration -- 12 B per element on the
                iterations that read C, 8 B on the others, 12 B for the final
-               unfold) over its measured time, against the measured HBM copy
-               bandwidth; x_update_10000 inside it: the single-instance fused
-               X-update at 10000^2 (X + C = 800 MB, HBM resident), 400
-               iterations.
+               unfold -- times the share that an ncu capture saw in DRAM)
+               over its time against the measured copy bandwidth, its FP32
+               operations against the FP32 pipe at the sampled clock, and the
+               rate at which a streaming kernel would have to move its bytes;
+               x_update_10000 inside it: the single-instance fused X-update
+               at 10000^2 (X + C = 800 MB, HBM resident), 400 iterations.
   cpu_baseline the oracle (C restatement of the reference loop, OpenMP on
                every host core) solving instances of the same workload one
                at a time to the same stop -- forward only: the reference has
@@ -152,6 +155,16 @@ def solve_bytes(shapes, info, cbytes=4):
         tot += float(m) * n * ((8 + cbytes) * ((t + 1) // 2) + 8 * (t // 2) +
                                ((8 + cbytes) if r["converged"] else 0))
     return tot
+
+
+def solve_fp32_ops(shapes, info):
+    """FP32 additions, multiplications and fused multiply-adds of one batched QR
+    solve: per element 10 on the iterations that read C (two additions and the
+    fused -sC, three of the division, the fold, the objective, the row and the
+    column sum) and 7 on the others."""
+    return sum(float(m) * n * (10 * ((int(r["iters_run"]) + 1) // 2) +
+                               7 * (int(r["iters_run"]) // 2))
+               for (m, n), r in zip(shapes, info))
 
 
 # --------------------------------------------------------------------------- clocks
@@ -452,7 +465,6 @@ def batched_point(dev, flush, single_sample=16):
                         f"C = sq. Euclidean of N(0,I_8) clouds / max, uniform marginals, "
                         f"alpha={ALPHA}, rho={RHO}, relative eps {REL_EPS}"),
            "elements": int(elems.sum())}
-    peak, _ = measured_peak()
     for name, dtype in (("fp32", torch.float32), ("bf16_c", torch.bfloat16)):
         B = QRBatch(shapes, RHO, ALPHA, eps, device=dev)
         c = B.pack_c(costs, dtype=dtype)
@@ -480,7 +492,7 @@ def batched_point(dev, flush, single_sample=16):
         out[name] = {"solves_per_s": len(shapes) / t, "s_per_batch": t, "cols_per_tile": cpt,
                      "converged": int(sum(r["converged"] for r in info)),
                      "n_iter_min_median_max": [int(it.min()), float(np.median(it)), int(it.max())],
-                     "achieved_GBps": nbytes / t / 1e9, "frac_of_measured_hbm": nbytes / t / 1e9 / peak}
+                     "streaming_equivalent_GBps": nbytes / t / 1e9}
         del B, c, x, graph
     # The same instances one solve at a time (a sample, every 16th instance).
     ks = list(range(0, len(shapes), max(1, len(shapes) // single_sample)))
@@ -788,16 +800,27 @@ def run_gpu(args):
     ksec = statistics.mean(solve_s)
     ratio = profile_value("batch_resident_diff16.md", "traffic_over_algorithmic")
     hbm = hbm_point(dev, flush)
-    # The algorithmic bytes are those of streaming every active instance once
-    # per iteration; on resident tiles few of them reach HBM (traffic).
-    roofline = {"bound": "latency, L2 and shared memory",
+    # On resident tiles few of the bytes that streaming would move reach HBM: the
+    # fractions are of what the launch does move (frac) and of the FP32 pipe that
+    # its steps keep busy (fp32_pipe); streaming_equivalent compares it with a
+    # launch that streams every active instance once per iteration.
+    moved = ratio * kbytes if ratio else None
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    mhz = clk.summary().get("sm_mhz")
+    ops = solve_fp32_ops(shapes, info)
+    pipe = sms * 128 * mhz * 1e6 if mhz else None
+    roofline = {"bound": "latency, the FP32 and shared-memory pipes and L2",
                 "kernel": "drot_resident_batch_kernel<QR, float>",
-                "achieved": kbytes / ksec / 1e9, "peak": peak, "unit": "GB/s",
-                "frac": kbytes / ksec / 1e9 / peak, "peak_source": peak_kind,
-                "traffic": ratio * kbytes if ratio else None,
-                "algorithmic_bytes_per_launch": kbytes,
-                "traffic_basis": ("ncu DRAM bytes / algorithmic bytes of a 16-instance capture "
-                                  "of the same kernel, times this launch's algorithmic bytes"),
+                "achieved": moved / ksec / 1e9 if moved else None, "peak": peak, "unit": "GB/s",
+                "frac": moved / ksec / 1e9 / peak if moved else None, "peak_source": peak_kind,
+                "traffic": moved,
+                "traffic_basis": ("ncu DRAM bytes / bytes of streaming, of a 16-instance capture "
+                                  "of the same kernel, times this launch's bytes of streaming"),
+                "fp32_pipe": {"achieved": ops / ksec / 1e12, "unit": "T operations/s",
+                              "peak": pipe / 1e12 if pipe else None,
+                              "frac": ops / ksec / pipe if pipe else None},
+                "streaming_equivalent": {"algorithmic_bytes_per_launch": kbytes,
+                                         "GBps": kbytes / ksec / 1e9},
                 "x_update_10000": {"achieved": hbm["achieved_GBps"],
                                    "frac": hbm["achieved_GBps"] / peak,
                                    "us_per_iteration": hbm["us_per_iteration"]}}

@@ -50,7 +50,9 @@ typedef struct {
                           last stop test (-1 if none ran) */
   double phase_ms[4];  /* device time of the solve split by stage, summed over
                           iterations: fused X-update, first grid barrier,
-                          dual update, second grid barrier + stop test */
+                          dual update, second grid barrier + stop test (on
+                          resident tiles: X-update; sums, exchange and duals;
+                          barrier; stop test) */
 } drot_result;
 
 /* Storage types of the cost matrix C for the *_ex entry points.  Iterates

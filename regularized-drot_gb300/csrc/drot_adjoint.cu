@@ -165,11 +165,10 @@ __global__ void adj_mask_kernel(const AdjParams A) {
 // the first MMA's k, then the second's) of thread-in-group t holds bits 4 t + r
 // and 4 t + r + 16, as the FP16 numbers 2^(r - 24); the digits carry 2^-r.
 //
-// us per CG iteration, bits walked -> here: 8 instances of 512..2048 rows and
-// columns with a tenth of the entries on the support 134 -> 17 (0.1 %: 119 ->
-// 17), one of 200 28 -> 12, 64 of 512..4096 715 -> 227 (0.1 %: 241 -> 225).  Of
-// the 8 instances' 32,000 clocks the MMAs take about 6000, the digits 2000, the
-// staged direction 3000, the scalars and sums 12,000 and two grid barriers 8000.
+// us per CG iteration (a solve's time over its iterations), bits walked -> here: 8
+// instances of 512..2048 rows and columns with 0.5 % of the entries on the support
+// 89 -> 19, with 0.15 % 101 -> 18; one of 200 x 200 35 -> 18; 64 of 512..4096 with
+// 1 % 257 -> 133.
 constexpr int kAdjThreads = 512;
 constexpr int kAdjChunk = 4096;     // entries whose digits are staged at a time, at most
 constexpr int kAdjBlock = 512;      // lines whose sums are held at a time

@@ -263,10 +263,11 @@ static size_t cost_smem_bytes(int dim) {
 //     the d components of two columns over its share of the band's rows (x
 //     broadcast), the shares are added -> the band's partial of dL/dy.
 // A second kernel adds the partials in order.  No atomics: deterministic.
-// Bound by the FP32 pipe (2 (d + 1) FMAs per element) and the 8 B per element
-// of G and C about alike at d = 16.  One CTA per band walking all columns,
-// which this replaces, kept 16 CTAs busy on a 4000 x 3000 matrix: 900 us
-// against 47 us here.
+// Bound at d = 16 by issue slots and shared memory, about half busy each (2 (d +
+// 1) FMAs per element; 90 M elements: 51 % and 43 %, DRAM at 0.43 of the copy
+// bandwidth), and by the latency of a tile's loads between its barriers.  One CTA
+// per band walking all columns, which this replaces, kept 16 CTAs busy on a 4000
+// x 3000 matrix: 900 us against 47 us here.
 
 constexpr int kGradRows = 256;   // rows per band (= threads)
 constexpr int kGradCols = 32;    // columns per tile

@@ -6,11 +6,14 @@
 // a CTA owns one tile of X and C in shared memory for the whole solve, and per
 // iteration the CTAs exchange only the tiles' row and column sums.  Measured,
 // us per iteration, streaming -> here: QR 96 x 80 6.9 -> 2.6, 1000 x 1000 9.6
-// -> 3.3, 1500 x 1500 11.3 -> 4.1, 1850 x 1850 13.2 -> 5.7; GL 300 x 200 8.9
-// -> 3.3, 1500 x 1000 (2 classes) 12.1 -> 5.8.  Bound by latency: at 1000 x
-// 1000 an iteration of 6300 clocks has two 4-column steps of a warp (1800), the
-// sums over warps and the duals (about 1500), one exchange through L2 (2000)
-// and the divisions by the row and column counts (400).
+// -> 3.1, 1500 x 1500 11.3 -> 4.1, 1850 x 1850 13.2 -> 5.7; GL 300 x 200 8.9
+// -> 3.3, 1500 x 1000 (2 classes) 12.1 -> 5.8.  Bound by latency; the stages of
+// CTA 0, as the kernel times them (drot_result.phase_ms), us per iteration:
+//                          X-update   sums, exchange, duals   barrier   stop test
+//   QR 96 x 80 (one CTA)     1.5              0.6               0.3        0.1
+//   QR 1000 x 1000           1.2              1.3               0.4        0.1
+//   GL 1500 x 1000           2.0              3.2               0.7        0.1
+//   QR 3000 x 3000           7.4              2.6               0.7        0.7
 //
 // Tiles.  The grid is GR x GC CTAs, at most one per SM.  CTA (br, bc) owns the
 // rows of band br (QR: equal heights, multiples of 4; GL: one class) and an
@@ -44,8 +47,11 @@
 // read round r.  Measured, one exchange of 152 CTAs in 8 x 19 tiles of 128 x
 // 53: 2000 cycles; with tagged words that each reader sums itself 5900, with
 // a counter barrier and loads after it 5500.
-//   Fixed point: a total has an error of at most GC 2^-47, below the rounding
-// of the FP32 duals it updates.  A CTA whose mass would exceed the words'
+//   Fixed point: a total has an error of at most GC 2^-47, an absolute one beside a
+// mass of about 1: below the FP32 rounding of sums and duals above GC 2^-23.  Rows
+// of smaller marginals keep fewer bits of their sums than FP32 has; the errors of
+// plans and duals against 64 bits, marginals of 1e-8 and 1e-11 and cold starts
+// included, are the streaming kernel's (its sums of a warp are float, too).  A CTA whose mass would exceed the words'
 // range (or is not finite) adds a poison count to the mass word instead; then
 // every CTA repeats the round with 8 fraction bits fewer (or, where all finite
 // sums fit, adds a round of counts of infinities and NaNs), so the arithmetic
